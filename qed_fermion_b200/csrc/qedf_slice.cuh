@@ -347,11 +347,14 @@ struct Slice {
   }
 
   // BUF: exchange buffer 0 or 1 fixed at compile time, or -1 for the
-  // alternating run-time choice
+  // alternating run-time choice.  The shuffle variant always alternates at run
+  // time: its x-bond factors use no buffer, so by BUF alone the four y-bond
+  // factors of B would share one buffer with a single barrier each, and a warp
+  // could overwrite values that a slower warp still has to read.
   template <int G, int MODE, int BUF = -1>
   __device__ __forceinline__ void factor(Cx<R> (&v)[BY][2]) {
     const R c = (G == 0) ? c1 : ch;
-    Cx<R>* buf = BUF >= 0 ? xb[BUF] : (cur ? xb[1] : xb[0]);
+    Cx<R>* buf = (!XS && BUF >= 0) ? xb[BUF] : (cur ? xb[1] : xb[0]);
     if (XS && (G == 0 || G == 2)) {
       // neighbours' old values by shuffle; every lane takes part
 #pragma unroll
@@ -440,7 +443,7 @@ struct Slice {
         v[0][CC] = nt;
       }
     }
-    if (BUF < 0) cur ^= 1;
+    if (XS || BUF < 0) cur ^= 1;
   }
 
   // B = F4 F3 F2 F1 F2 F3 F4 without the scalar Cb (FAC_TILDE) or exact.
