@@ -16,8 +16,7 @@ struct OpArgs {
   void* z;          // output vectors
   int L, Nt, bs;
   int rhs_per_phi;  // consecutive vectors sharing one angle array
-  int T;            // slab length (0 = auto)
-  int xs;           // allow the warp-shuffle engine (single precision, L <= 64)
+  int T;            // slab length (0 = one contiguous run of slices per block)
   double c1, ch, t1, th, Cb;
 };
 
@@ -43,7 +42,8 @@ struct ForceArgs {
   const void* xi;
   void* F;
   int L, Nt, bs, rhs_per_phi, T;
-  double c1, ch, t1, th;
+  double t1, th, Cb;
+  double kappa[7];  // scalars of the force terms at the seven factor positions (k_force)
 };
 
 struct BosonArgs {

@@ -14,143 +14,204 @@
 namespace qedf {
 
 // ============================================================================
-// M, M^dagger, M^dagger M over tau-slabs
+// M, M^dagger, M^dagger M
 // ============================================================================
 //
-// One thread block handles one right-hand side and one slab [a, b) of output
-// slices.  With x_t the slices of the input and sigma_t = +1 (t < Nt-1) or -1
+// With x_t the slices of the input and sigma_t = +1 (t < Nt-1) or -1
 // (t = Nt-1):
 //   (M x)_t      = x_t - sigma_{t-1} B_{t-1} x_{t-1}
 //   (M^dag y)_t  = y_t - sigma_t B_t y_{t+1}
 //   (M^dag M x)_t: y = M x is produced slice by slice in registers and M^dag
 //                  applied to it, so x is read once and one extra slice of y
-//                  (the slab's lower halo) is recomputed.
-template <typename R, typename A, int BY, int OP, int EC>
-__global__ void __launch_bounds__(MaxT<BY, EC>::value, MaxT<BY, EC>::min_blocks) k_operator(OpArgs p) {
+//                  (the run's lower halo) is recomputed.
+// The slices of all right-hand sides form one line that is cut into one
+// contiguous run per block (block_run), so every SM gets the same number of
+// slices; with a slab length, a run is one slab instead.  Measured with the
+// engine of qedf_slice.cuh at 8 right-hand sides, L = 48, Ltau = 480: 57 us
+// complex64 (73 with fixed slabs and one block per SM) and 187 us complex128
+// (328); the algorithmic bytes take 32 and 65 us at the copy bandwidth.  What
+// is left is issue slots (53 % busy) and shared-memory wavefronts (58 %); in
+// double precision the FP64 pipe, half of it for the phases' sincos.
+//
+// CFG_TALL (double precision, tall tiles with many threads): the phases live
+// in the thread's record, there is one exchange buffer, and y_t waits in z's
+// own slice instead of a stash, so that 384 or 512 threads fit in shared
+// memory and registers.  2 x 2 double tiles also leave y_t in z, and fetch the
+// next slice's angles by cp.async into the stash instead (185 against 189 us at
+// L = 48, 95 against 107 at L = 36: no spills; in single precision the same
+// costs 8 to 15 %, the shared-memory pipe being the busy one there).
+enum { CFG_REG = 0, CFG_TALL = 1 };
+
+// threads and resident blocks that an operator kernel is compiled for
+template <typename R, int BY, int CFG>
+struct OpT {
+  // 2 x 4 double tiles keep 168 registers (384 threads) unless CFG_TALL
+  static constexpr int threads = (sizeof(R) == 8 && BY == 4 && CFG == CFG_REG) ? 384 : MaxT<R, BY>::value;
+  static constexpr int min_blocks = MaxT<R, BY>::min_blocks;
+};
+
+// first and one-past-last global slice (right-hand side * Nt + t) of a block
+__device__ __forceinline__ void block_run(int bs, int Nt, int T, int64_t& w0, int64_t& w1) {
+  if (T > 0) {
+    const int per = (Nt + T - 1) / T, rb = blockIdx.x / per, k = blockIdx.x % per;
+    w0 = (int64_t)rb * Nt + (int64_t)k * T;
+    w1 = min(w0 + T, (int64_t)(rb + 1) * Nt);
+  } else {
+    const int64_t W = (int64_t)bs * Nt;
+    w0 = W * blockIdx.x / gridDim.x;
+    w1 = W * (blockIdx.x + 1) / gridDim.x;
+  }
+}
+
+template <typename R, typename A, int BY, int OP, int CFG>
+__global__ void __launch_bounds__(OpT<R, BY, CFG>::threads, OpT<R, BY, CFG>::min_blocks) k_operator(OpArgs p) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr bool PHS = (EC & EC_PHS) != 0;
-  constexpr bool STASH = (EC & EC_NOSTASH) == 0;
-  constexpr bool XS = (EC & EC_XS) != 0;
-  constexpr int LT = ec_fixed_l(EC);
-  Slice<R, BY, PHS, XS, LT> S;
-  const int L = lattice_l<EC>(p.L);
-  S.init(L, smem, 2, (R)p.c1, (R)p.ch, threadIdx.x);
-  const int Vs = L * L;
-  const size_t sv = 2 * (size_t)Vs;  // reals per slice (vector and angles)
-  const int rb = blockIdx.y;
-  const int a = blockIdx.x * p.T;
-  const int b = min(a + p.T, p.Nt);
-  const A* phi = reinterpret_cast<const A*>(p.phi) + (size_t)(rb / p.rhs_per_phi) * p.Nt * sv;
-  const R* x = reinterpret_cast<const R*>(p.x) + (size_t)rb * p.Nt * sv;
-  R* z = reinterpret_cast<R*>(p.z) + (size_t)rb * p.Nt * sv;
+  constexpr bool TALL = CFG == CFG_TALL;
+  // angles of the next slice wait in registers where these allow it
+  constexpr bool PF = sizeof(R) == 4 && BY >= 4;
+  using Eng = Slice<R, BY, TALL, TALL ? 1 : 2>;
+  Eng S;
+  S.init(p.L, smem, threadIdx.x);
+  // where y_t and the next slice's angles wait (OP_MHM; see above)
+  constexpr bool STAGE = OP == OP_MHM && sizeof(R) == 8 && BY == 2;
+  constexpr bool IN_Z = TALL || STAGE;
+  Stash<R, BY> st;
+  if constexpr (OP == OP_MHM && !TALL) st.init(smem + slice_smem<R>(blockDim.x, Eng::REC), threadIdx.x);
+  const size_t sv = 2 * (size_t)p.L * p.L;  // reals per slice (vector and angles)
   const R t1 = (R)p.t1, th = (R)p.th, Cb = (R)p.Cb;
   const int Nt = p.Nt;
-  // Three blocks live in registers; y_t waits in the thread-private stash
-  // (or in a fourth register block when there is no stash).
-  Cx<R> X0[BY][2], X1[BY][2], Y[BY][2];
-  Cx<R> Yp[STASH ? 1 : BY][2];
-
-  if (OP == OP_M) {
-    int tp = (a - 1 + Nt) % Nt;
-    if (S.on) S.load(X0, x + tp * sv);
-    for (int t = a; t < b; ++t) {
-      if (S.on) S.load(X1, x + t * sv);
-      S.phases(phi + tp * sv, t1, th);
-      S.template applyB<FAC_TILDE>(X0);
-      if (S.on) {
-        axpy_blk<R, BY>(Y, X1, sigma_of<R>(tp, Nt) * Cb, X0);
-        S.store(z + t * sv, Y);
+  int64_t w, w1;
+  block_run(p.bs, Nt, p.T, w, w1);
+  while (w < w1) {
+    const int rb = (int)(w / Nt), a = (int)(w - (int64_t)rb * Nt), b = (int)min((int64_t)Nt, a + (w1 - w));
+    w += b - a;
+    const A* phi = reinterpret_cast<const A*>(p.phi) + (size_t)(rb / p.rhs_per_phi) * Nt * sv;
+    const R* x = reinterpret_cast<const R*>(p.x) + (size_t)rb * Nt * sv;
+    R* z = reinterpret_cast<R*>(p.z) + (size_t)rb * Nt * sv;
+    Cx<R> X0[BY][2], X1[BY][2];
+    A ang[BY][4];
+    if constexpr (OP == OP_M) {
+      int tp = a == 0 ? Nt - 1 : a - 1;
+      S.load(X0, x + tp * sv);
+      if (PF) S.load_angles(ang, phi + tp * sv);
+      for (int t = a; t < b; ++t) {
+        if (!PF) S.load_angles(ang, phi + tp * sv);
+        S.load(X1, x + t * sv);
+        S.phases(ang, t1, th);
+        if (PF && t + 1 < b) S.load_angles(ang, phi + t * sv);
+        if ((t - a) & 1) S.template applyB<1>(X0);
+        else S.template applyB<0>(X0);
+        axpy_blk<R, BY>(X0, X1, sigma_of<R>(tp, Nt) * Cb, X0);
+        S.store(z + t * sv, X0);
+        copy_blk<R, BY>(X0, X1);
+        tp = t;
       }
-      copy_blk<R, BY>(X0, X1);
-      tp = t;
-    }
-  } else if (OP == OP_MH) {
-    if (S.on) S.load(X0, x + a * sv);
-    for (int t = a; t < b; ++t) {
-      const int tn = (t + 1) % Nt;
-      if (S.on) S.load(X1, x + tn * sv);
-      S.phases(phi + t * sv, t1, th);
-      copy_blk<R, BY>(Y, X1);
-      S.template applyB<FAC_TILDE>(Y);
-      if (S.on) {
+    } else if constexpr (OP == OP_MH) {
+      S.load(X0, x + a * sv);
+      if (PF) S.load_angles(ang, phi + a * sv);
+      for (int t = a; t < b; ++t) {
+        const int tn = t + 1 == Nt ? 0 : t + 1;
+        if (!PF) S.load_angles(ang, phi + t * sv);
+        S.load(X1, x + tn * sv);
+        S.phases(ang, t1, th);
+        if (PF && t + 1 < b) S.load_angles(ang, phi + (t + 1) * sv);
+        Cx<R> Y[BY][2];
+        copy_blk<R, BY>(Y, X1);
+        if ((t - a) & 1) S.template applyB<1>(Y);
+        else S.template applyB<0>(Y);
         axpy_blk<R, BY>(Y, X0, sigma_of<R>(t, Nt) * Cb, Y);
         S.store(z + t * sv, Y);
+        copy_blk<R, BY>(X0, X1);
       }
-      copy_blk<R, BY>(X0, X1);
-    }
-  } else {  // OP_MHM
-    // prologue: y_a = x_a - sigma_{a-1} B_{a-1} x_{a-1}
-    const int tp = (a - 1 + Nt) % Nt;
-    if (S.on) {
+    } else {  // OP_MHM
+      Cx<R> Y[BY][2];
+      const int tp = a == 0 ? Nt - 1 : a - 1;
       S.load(X0, x + tp * sv);
+      S.load_angles(ang, phi + tp * sv);
       S.load(X1, x + a * sv);
-    }
-    A ang[BY][4];
-    if constexpr (!PHS) S.load_angles(ang, phi + a * sv);
-    S.phases(phi + tp * sv, t1, th);
-    S.template applyB<FAC_TILDE>(X0);
-    axpy_blk<R, BY>(Y, X1, sigma_of<R>(tp, Nt) * Cb, X0);
-    if constexpr (STASH) S.park(Y); else copy_blk<R, BY>(Yp, Y);
-    copy_blk<R, BY>(X0, X1);
-    for (int t = a; t < b; ++t) {
-      const int tn = (t + 1) % Nt;
-      if (S.on) S.load(X1, x + tn * sv);
-      if constexpr (!PHS) {
-        // phases of slice t from angles fetched one slice ahead
-        S.phases_from(ang, t1, th);
-        if (t + 1 < b) S.load_angles(ang, phi + (t + 1) * sv);
-      } else {
-        S.phases(phi + t * sv, t1, th);
-      }
-      const R sg = sigma_of<R>(t, Nt) * Cb;
-      S.template applyB<FAC_TILDE>(X0);          // B_t x_t
-      axpy_blk<R, BY>(Y, X1, sg, X0);             // y_{t+1}
-      if constexpr (STASH) {
-        S.unpark(X0);                             // y_t
-        S.park(Y);
-      } else {
-        copy_blk<R, BY>(X0, Yp);
-        copy_blk<R, BY>(Yp, Y);
-      }
-      S.template applyB<FAC_TILDE, 1>(Y);         // B_t y_{t+1}
-      if (S.on) {
-        axpy_blk<R, BY>(Y, X0, sg, Y);            // z_t = y_t - sigma_t B_t y_{t+1}
-        S.store(z + t * sv, Y);
-      }
+      S.phases(ang, t1, th);
+      if (PF) S.load_angles(ang, phi + a * sv);
+      if constexpr (STAGE) S.fetch_angles(st, phi + a * sv);
+      S.template applyB<0>(X0);
+      axpy_blk<R, BY>(Y, X1, sigma_of<R>(tp, Nt) * Cb, X0);  // y_a
+      if constexpr (IN_Z) S.store(z + a * sv, Y); else st.park(Y);
       copy_blk<R, BY>(X0, X1);
+      for (int t = a; t < b; ++t) {
+        const int tn = t + 1 == Nt ? 0 : t + 1;
+        if constexpr (STAGE) S.take_angles(ang, st);
+        else if (!PF) S.load_angles(ang, phi + t * sv);
+        S.load(X1, x + tn * sv);
+        S.phases(ang, t1, th);
+        if (t + 1 < b) {
+          if constexpr (STAGE) S.fetch_angles(st, phi + (t + 1) * sv);
+          else if (PF) S.load_angles(ang, phi + (t + 1) * sv);
+        }
+        const R sg = sigma_of<R>(t, Nt) * Cb;
+        S.template applyB<1>(X0);             // B_t x_t
+        axpy_blk<R, BY>(Y, X1, sg, X0);       // y_{t+1}
+        if constexpr (IN_Z) {
+          if (t + 1 < b) S.store(z + (t + 1) * sv, Y);
+        } else {
+          st.unpark(X0);                      // y_t
+          st.park(Y);
+        }
+        S.template applyB<0>(Y);              // B_t y_{t+1}
+        if constexpr (IN_Z) S.load_st(X0, z + t * sv);
+        axpy_blk<R, BY>(Y, X0, sg, Y);        // z_t = y_t - sigma_t B_t y_{t+1}
+        S.store(z + t * sv, Y);
+        copy_blk<R, BY>(X0, X1);
+      }
     }
+    // the next run's first factor uses buffer 0, as may this run's last
+    __syncthreads();
   }
 }
 
 // ============================================================================
 // b_vec_per_tau: B_t v or its six partial products, one slice
 // ============================================================================
-template <typename R, typename A, int BY, bool PHS>
-__global__ void __launch_bounds__(MaxThreads<BY>::value, 1) k_bvec(BvecArgs p) {
+template <typename R, typename A, int BY>
+__global__ void __launch_bounds__(MaxT<R, BY>::value, 1) k_bvec(BvecArgs p) {
   extern __shared__ __align__(16) unsigned char smem[];
-  Slice<R, BY, PHS> S;
-  S.init(p.L, smem, 2, (R)p.c1, (R)p.ch, threadIdx.x);
+  Slice<R, BY> S;
+  S.init(p.L, smem, threadIdx.x);
   const size_t sv = 2 * (size_t)p.L * p.L;
-  const A* phi = reinterpret_cast<const A*>(p.phi);
   const R* v = reinterpret_cast<const R*>(p.v) + blockIdx.x * sv;
   R* out = reinterpret_cast<R*>(p.out) + blockIdx.x * sv * (p.interm ? 6 : 1);
   Cx<R> W[BY][2];
-  if (S.on) S.load(W, v);
-  S.phases(phi, (R)p.t1, (R)p.th);
-  S.template factor<3, FAC_TRUE>(W);
-  if (p.interm && S.on) S.store(out + 0 * sv, W);
-  S.template factor<2, FAC_TRUE>(W);
-  if (p.interm && S.on) S.store(out + 1 * sv, W);
-  S.template factor<1, FAC_TRUE>(W);
-  if (p.interm && S.on) S.store(out + 2 * sv, W);
-  S.template factor<0, FAC_TRUE>(W);
-  if (p.interm && S.on) S.store(out + 3 * sv, W);
-  S.template factor<1, FAC_TRUE>(W);
-  if (p.interm && S.on) S.store(out + 4 * sv, W);
-  S.template factor<2, FAC_TRUE>(W);
-  if (p.interm && S.on) S.store(out + 5 * sv, W);
-  S.template factor<3, FAC_TRUE>(W);
-  if (!p.interm && S.on) S.store(out, W);
+  S.load(W, v);
+  S.phases_of(reinterpret_cast<const A*>(p.phi), (R)p.t1, (R)p.th);
+  R scale = 1;  // the product of the applied factors' cosh
+  auto put = [&](R* to) {
+    if (!S.on) return;
+#pragma unroll
+    for (int r = 0; r < BY; ++r) st2(to + S.off + r * S.rs, scale * W[r][0], scale * W[r][1]);
+  };
+  const R c1 = (R)p.c1, ch = (R)p.ch;
+  S.template factor<3, 0>(W);
+  scale *= ch;
+  if (p.interm) put(out);
+  S.template factor<2, 1>(W);
+  scale *= ch;
+  if (p.interm) put(out + 1 * sv);
+  S.template factor<1, 0>(W);
+  scale *= ch;
+  if (p.interm) put(out + 2 * sv);
+  S.template factor<0, 1>(W);
+  scale *= c1;
+  if (p.interm) put(out + 3 * sv);
+  S.template factor<1, 0>(W);
+  scale *= ch;
+  if (p.interm) put(out + 4 * sv);
+  S.template factor<2, 1>(W);
+  scale *= ch;
+  if (p.interm) {
+    put(out + 5 * sv);
+  } else {
+    S.template factor<3, 0>(W);
+    scale *= ch;
+    put(out);
+  }
 }
 
 // ============================================================================
@@ -317,177 +378,148 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_precon_band(Pre
 // while l is advanced forwards, so no partial product is stored.  This is the
 // sum that the reference evaluates with explicit partial products
 // (force_f_fast, hmc_sampler_batch.py:2150-2227; force_f_sparse :2230-2330).
-template <typename R, typename A, int BY, bool PHS, int LT = 0>
-struct ForceSlice {
-  using Eng = Slice<R, BY, PHS, false, LT>;
-  Eng& S;
-  __device__ ForceSlice(Eng& s) : S(s) {}
+//
+// The factors are applied without their scalars c_j, backwards as I - tK
+// ((I - tK)(I + tK) = I / c^2), so at position k the bond terms carry
+// kappa_k = 2 Cb prod_{j<=k} c_j^2.  The exchange is the engine's: a cross bond's owner
+// exports conj(a) R_i and conj(a) l_i and gets R_j and l_j, which is all that
+// its own force term and both updates need.  Every slice is independent of
+// the others: the slices of all right-hand sides are dealt as block_run does.
+// Measured, 2 right-hand sides at L = 48, Ltau = 480, complex64:
+// 31 us, against 39 with fixed slabs and an engine that exchanged both vectors and phases.
+template <typename R, int BY>
+struct ForceT {
+  static constexpr int threads = MaxT<R, BY>::value;
+};
 
-  // term for one bond: c * [conj(l_i) (i a) R_j + conj(l_j) conj(i a) R_i]
-  __device__ static __forceinline__ R term(Cx<R> li, Cx<R> lj, Cx<R> Ri, Cx<R> Rj, Cx<R> a, R c) {
-    const Cx<R> ia = mk<R>(-a.im, a.re);
-    const Cx<R> u = cjmul(li, cmul(ia, Rj));
-    const Cx<R> w = cjmul(lj, cjmul(ia, Ri));
-    return (R)2 * c * (u.re + w.re);
+template <typename R, int BY>
+struct ForceSlice : Slice<R, BY, false, 2, 2> {
+  using Base = Slice<R, BY, false, 2, 2>;
+
+  // kappa-free term of one bond, R after the factor's inverse, l before it:
+  // Re[conj(l_i) (i a) R_j + conj(l_j) conj(i a) R_i]
+  __device__ static __forceinline__ R term(Cx<R> li, Cx<R> lj, Cx<R> Ri, Cx<R> Rj, Cx<R> a) {
+    // X = conj(l_i) R_j, Y = conj(l_j) R_i
+    const R d1 = fma(lj.re, Ri.im, fma(-lj.im, Ri.re, fma(-li.re, Rj.im, li.im * Rj.re)));  // Im Y - Im X
+    const R d2 = fma(lj.re, Ri.re, fma(lj.im, Ri.im, fma(li.re, Rj.re, li.im * Rj.im)));    // Re X + Re Y
+    return fma(a.re, d1, -(a.im * d2));
+  }
+  // a bond inside the tile
+  __device__ static __forceinline__ void local(Cx<R>& Ri, Cx<R>& Rj, Cx<R>& li, Cx<R>& lj, Cx<R> a, R kap, R& F) {
+    Base::pair(Ri, Rj, mk<R>(-a.re, -a.im));
+    F = fma(kap, term(li, lj, Ri, Rj, a), F);
+    Base::pair(li, lj, a);
   }
 
-  // one factor position: R <- F_g^{-1} R, accumulate force, l <- F_g l.
-  // Uses exchange buffers 2*par, 2*par+1 (par alternates per call).
-  template <int G>
-  __device__ __forceinline__ void step(Cx<R> (&Rv)[BY][2], Cx<R> (&l)[BY][2], R (&Fx)[BY][2],
-                                       R (&Fy)[BY][2], int par) {
-    const R c = (G == 0) ? S.c1 : S.ch;
-    Cx<R>* bR = S.xb[2 * par];
-    Cx<R>* bl = S.xb[2 * par + 1];
-    if (G == 0 || G == 2) {
-      // cross row r uses slots r & ~1 (left column) and (r & ~1) + 1 (right column)
-      if (S.on) {
+  // one factor position: R <- (I - K_g) R, accumulate the force, l <- (I + K_g) l
+  template <int G, int BUF>
+  __device__ __forceinline__ void step(Cx<R> (&Rv)[BY][2], Cx<R> (&l)[BY][2], R (&Fx)[BY][2], R (&Fy)[BY][2],
+                                       R kap) {
+    constexpr int B0 = BUF * 2 * BY, B1 = B0 + BY;  // exchange slots of R and l
+    Cx<R>* me = this->me;
+    if constexpr (G == 0 || G == 2) {
+      constexpr int RC = G == 0 ? 1 : 0;
 #pragma unroll
-        for (int r = 0; r < BY; ++r)
-          if (Eng::xcross(G, r)) {
-            S.slot(bR, r & ~1)[S.id] = Rv[r][0];
-            S.slot(bR, (r & ~1) + 1)[S.id] = Rv[r][1];
-            S.slot(bl, r & ~1)[S.id] = l[r][0];
-            S.slot(bl, (r & ~1) + 1)[S.id] = l[r][1];
-          }
+      for (int r = RC; r < BY; r += 2) {
+        const int q = r & ~1;
+        me[B0 + q] = Rv[r][0];
+        me[B0 + q + 1] = Base::cjm(this->px(r, 1), Rv[r][1]);
+        me[B1 + q] = l[r][0];
+        me[B1 + q + 1] = Base::cjm(this->px(r, 1), l[r][1]);
       }
-      __syncthreads();
-      if (!S.on) return;
 #pragma unroll
-      for (int r = 0; r < BY; ++r) {
-        if (!Eng::xcross(G, r)) {
-          const Cx<R> a = S.TPX(r, 0);
-          const Cx<R> Ri = Rv[r][0], Rj = Rv[r][1];
-          const Cx<R> nRi = c * cfma(cneg(a), Rj, Ri);
-          const Cx<R> nRj = c * cjfma(cneg(a), Ri, Rj);
-          Fx[r][0] += term(l[r][0], l[r][1], nRi, nRj, a, c);
-          const Cx<R> li = l[r][0], lj = l[r][1];
-          l[r][0] = c * cfma(a, lj, li);
-          l[r][1] = c * cjfma(a, li, lj);
-          Rv[r][0] = nRi;
-          Rv[r][1] = nRj;
-        } else {
-          const Cx<R> Rright = S.slot(bR, r & ~1)[S.idr], lright = S.slot(bl, r & ~1)[S.idr];
-          const Cx<R> Rleft = S.slot(bR, (r & ~1) + 1)[S.idl], lleft = S.slot(bl, (r & ~1) + 1)[S.idl];
-          // pair (i = own x0+1, j = right neighbour's x0), phase own
-          const Cx<R> a = S.TPX(r, 1);
-          const Cx<R> nRi = c * cfma(cneg(a), Rright, Rv[r][1]);
-          const Cx<R> nRj = c * cjfma(cneg(a), Rv[r][1], Rright);
-          Fx[r][1] += term(l[r][1], lright, nRi, nRj, a, c);
-          // pair (i = left neighbour's x0+1, j = own x0), phase from the left
-          const Cx<R> al = S.TPL(r);
-          const Cx<R> nR0 = c * cjfma(cneg(al), Rleft, Rv[r][0]);
-          const Cx<R> nl0 = c * cjfma(al, lleft, l[r][0]);
-          const Cx<R> nl1 = c * cfma(a, lright, l[r][1]);
-          Rv[r][1] = nRi;
-          Rv[r][0] = nR0;
-          l[r][1] = nl1;
-          l[r][0] = nl0;
-        }
+      for (int r = 1 - RC; r < BY; r += 2)
+        local(Rv[r][0], Rv[r][1], l[r][0], l[r][1], this->px(r, 0), kap, Fx[r][0]);
+      __syncthreads();
+#pragma unroll
+      for (int r = RC; r < BY; r += 2) {
+        const int q = r & ~1;
+        const Cx<R> a = this->px(r, 1);
+        edge(Rv[r][1], l[r][1], this->rt[B0 + q], this->rt[B1 + q], a, kap, Fx[r][1]);
+        Rv[r][0] = Rv[r][0] - this->lf[B0 + q + 1];
+        l[r][0] = l[r][0] + this->lf[B1 + q + 1];
       }
     } else {
-      constexpr int CL = (G == 1) ? 0 : 1;
-      constexpr int CC = 1 - CL;
-      if (S.on) {
-        S.slot(bR, 0)[S.id] = Rv[0][CC];
-        S.slot(bR, 1)[S.id] = Rv[BY - 1][CC];
-        S.slot(bl, 0)[S.id] = l[0][CC];
-        S.slot(bl, 1)[S.id] = l[BY - 1][CC];
-      }
+      constexpr int CL = (G == 1) ? 0 : 1, CC = 1 - CL;
+      const Cx<R> a = this->py(BY - 1, CC);
+      me[B0] = Rv[0][CC];
+      me[B0 + 1] = Base::cjm(a, Rv[BY - 1][CC]);
+      me[B1] = l[0][CC];
+      me[B1 + 1] = Base::cjm(a, l[BY - 1][CC]);
+#pragma unroll
+      for (int r = 0; r < BY; r += 2)
+        local(Rv[r][CL], Rv[r + 1][CL], l[r][CL], l[r + 1][CL], this->py(r, CL), kap, Fy[r][CL]);
+#pragma unroll
+      for (int r = 1; r + 1 < BY; r += 2)
+        local(Rv[r][CC], Rv[r + 1][CC], l[r][CC], l[r + 1][CC], this->py(r, CC), kap, Fy[r][CC]);
       __syncthreads();
-      if (!S.on) return;
-      // pairs fully inside the block
-#pragma unroll
-      for (int r = 0; r < BY; r += 2) {
-        const Cx<R> a = S.TPY(r, CL);
-        const Cx<R> Ri = Rv[r][CL], Rj = Rv[r + 1][CL];
-        const Cx<R> nRi = c * cfma(cneg(a), Rj, Ri);
-        const Cx<R> nRj = c * cjfma(cneg(a), Ri, Rj);
-        Fy[r][CL] += term(l[r][CL], l[r + 1][CL], nRi, nRj, a, c);
-        const Cx<R> li = l[r][CL], lj = l[r + 1][CL];
-        l[r][CL] = c * cfma(a, lj, li);
-        l[r + 1][CL] = c * cjfma(a, li, lj);
-        Rv[r][CL] = nRi;
-        Rv[r + 1][CL] = nRj;
-      }
-#pragma unroll
-      for (int r = 1; r + 1 < BY; r += 2) {
-        const Cx<R> a = S.TPY(r, CC);
-        const Cx<R> Ri = Rv[r][CC], Rj = Rv[r + 1][CC];
-        const Cx<R> nRi = c * cfma(cneg(a), Rj, Ri);
-        const Cx<R> nRj = c * cjfma(cneg(a), Ri, Rj);
-        Fy[r][CC] += term(l[r][CC], l[r + 1][CC], nRi, nRj, a, c);
-        const Cx<R> li = l[r][CC], lj = l[r + 1][CC];
-        l[r][CC] = c * cfma(a, lj, li);
-        l[r + 1][CC] = c * cjfma(a, li, lj);
-        Rv[r][CC] = nRi;
-        Rv[r + 1][CC] = nRj;
-      }
-      // bottom pair: i = own last row, j = lower neighbour's first row
-      const Cx<R> Rbelow = S.slot(bR, 0)[S.idd], lbelow = S.slot(bl, 0)[S.idd];
-      const Cx<R> Rabove = S.slot(bR, 1)[S.idu], labove = S.slot(bl, 1)[S.idu];
-      const Cx<R> ab = S.TPY(BY - 1, CC);
-      const Cx<R> at = S.TPT(CC);
-      const Cx<R> Rb = Rv[BY - 1][CC], lb = l[BY - 1][CC];
-      const Cx<R> Rt = Rv[0][CC], lt = l[0][CC];
-      const Cx<R> nRi = c * cfma(cneg(ab), Rbelow, Rb);
-      const Cx<R> nRj = c * cjfma(cneg(ab), Rb, Rbelow);
-      Fy[BY - 1][CC] += term(lb, lbelow, nRi, nRj, ab, c);
-      // top site is the j end of the upper neighbour's bond
-      Rv[0][CC] = c * cjfma(cneg(at), Rabove, Rt);
-      l[0][CC] = c * cjfma(at, labove, lt);
-      Rv[BY - 1][CC] = nRi;
-      l[BY - 1][CC] = c * cfma(ab, lbelow, lb);
+      edge(Rv[BY - 1][CC], l[BY - 1][CC], this->dn[B0], this->dn[B1], a, kap, Fy[BY - 1][CC]);
+      Rv[0][CC] = Rv[0][CC] - this->up[B0 + 1];
+      l[0][CC] = l[0][CC] + this->up[B1 + 1];
     }
+  }
+  // the owner's side of a cross bond: i is its own site, j the neighbour's
+  __device__ static __forceinline__ void edge(Cx<R>& Ri, Cx<R>& li, Cx<R> Rj, Cx<R> lj, Cx<R> a, R kap, R& F) {
+    Cx<R> nj = Rj;
+    Base::pair(Ri, nj, mk<R>(-a.re, -a.im));
+    F = fma(kap, term(li, lj, Ri, nj, a), F);
+    li = cfma(a, lj, li);
   }
 };
 
-template <typename R, typename A, int BY, bool PHS, int LT = 0>
-__global__ void __launch_bounds__(MaxThreads<BY>::value, 1) k_force(ForceArgs p) {
+template <typename R, typename A, int BY>
+__global__ void __launch_bounds__(ForceT<R, BY>::threads, 1) k_force(ForceArgs p) {
   extern __shared__ __align__(16) unsigned char smem[];
-  Slice<R, BY, PHS, false, LT> S;
-  const int L = LT ? LT : p.L;
-  S.init(L, smem, 4, (R)p.c1, (R)p.ch, threadIdx.x);
-  ForceSlice<R, A, BY, PHS, LT> FS(S);
-  const int Vs = L * L;
-  const size_t sv = 2 * (size_t)Vs;
-  const int rb = blockIdx.y;
-  const int a = blockIdx.x * p.T;
-  const int b = min(a + p.T, p.Nt);
+  ForceSlice<R, BY> S;
+  S.init(p.L, smem, threadIdx.x);
+  const size_t sv = 2 * (size_t)p.L * p.L;
   const int Nt = p.Nt;
-  const A* phi = reinterpret_cast<const A*>(p.phi) + (size_t)(rb / p.rhs_per_phi) * Nt * sv;
-  const R* xi = reinterpret_cast<const R*>(p.xi) + (size_t)rb * Nt * sv;
-  A* F = reinterpret_cast<A*>(p.F) + (size_t)rb * Nt * sv;
-  Cx<R> Rv[BY][2], l[BY][2], Xn[BY][2];
-  if (S.on) S.load(Rv, xi + a * sv);
-  for (int t = a; t < b; ++t) {
-    const int tn = (t + 1) % Nt;
-    if (S.on) S.load(Xn, xi + tn * sv);
-    S.phases(phi + t * sv, (R)p.t1, (R)p.th);
-    S.template applyB<FAC_TRUE>(Rv);  // R_7 = B_t xi_t
-    axpy_blk<R, BY>(l, Rv, sigma_of<R>(t, Nt), Xn);
+  const R t1 = (R)p.t1, th = (R)p.th, Cb = (R)p.Cb;
+  R kap[7];
+#pragma unroll
+  for (int k = 0; k < 7; ++k) kap[k] = (R)p.kappa[k];
+  int64_t w, w1;
+  block_run(p.bs, Nt, p.T, w, w1);
+  for (; w < w1; ++w) {
+    const int rb = (int)(w / Nt), t = (int)(w - (int64_t)rb * Nt), tn = t + 1 == Nt ? 0 : t + 1;
+    const A* phi = reinterpret_cast<const A*>(p.phi) + (size_t)(rb / p.rhs_per_phi) * Nt * sv;
+    const R* xi = reinterpret_cast<const R*>(p.xi) + (size_t)rb * Nt * sv;
+    A* F = reinterpret_cast<A*>(p.F) + ((size_t)rb * Nt + t) * sv;
+    Cx<R> Rv[BY][2], l[BY][2];
+    S.load(Rv, xi + t * sv);
+    S.phases_of(phi + t * sv, t1, th);
+    S.load(l, xi + tn * sv);
+    S.template factor<3, 0>(Rv);  // R_7 = B_t xi_t
+    S.template factor<2, 1>(Rv);
+    S.template factor<1, 0>(Rv);
+    S.template factor<0, 1>(Rv);
+    S.template factor<1, 0>(Rv);
+    S.template factor<2, 1>(Rv);
+    S.template factor<3, 0>(Rv);
+    const R sg = sigma_of<R>(t, Nt);
     R Fx[BY][2], Fy[BY][2];
 #pragma unroll
-    for (int r = 0; r < BY; ++r) Fx[r][0] = Fx[r][1] = Fy[r][0] = Fy[r][1] = 0;
+    for (int r = 0; r < BY; ++r)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        l[r][c] = mk<R>(fma(Cb, Rv[r][c].re, -sg * l[r][c].re), fma(Cb, Rv[r][c].im, -sg * l[r][c].im));
+        Fx[r][c] = Fy[r][c] = 0;
+      }
     // positions k = 1..7 of B = F4 F3 F2 F1 F2 F3 F4
-    // (exchange buffers 2/3 first: buffers 0/1 may still be read by the
-    //  last factor of applyB in slower threads)
-    FS.template step<3>(Rv, l, Fx, Fy, 1);
-    FS.template step<2>(Rv, l, Fx, Fy, 0);
-    FS.template step<1>(Rv, l, Fx, Fy, 1);
-    FS.template step<0>(Rv, l, Fx, Fy, 0);
-    FS.template step<1>(Rv, l, Fx, Fy, 1);
-    FS.template step<2>(Rv, l, Fx, Fy, 0);
-    FS.template step<3>(Rv, l, Fx, Fy, 1);
+    S.template step<3, 1>(Rv, l, Fx, Fy, kap[0]);
+    S.template step<2, 0>(Rv, l, Fx, Fy, kap[1]);
+    S.template step<1, 1>(Rv, l, Fx, Fy, kap[2]);
+    S.template step<0, 0>(Rv, l, Fx, Fy, kap[3]);
+    S.template step<1, 1>(Rv, l, Fx, Fy, kap[4]);
+    S.template step<2, 0>(Rv, l, Fx, Fy, kap[5]);
+    S.template step<3, 1>(Rv, l, Fx, Fy, kap[6]);
     if (S.on) {
 #pragma unroll
       for (int r = 0; r < BY; ++r) {
         A o[4] = {(A)Fx[r][0], (A)Fy[r][0], (A)Fx[r][1], (A)Fy[r][1]};
-        st4(F + t * sv + 2 * ((S.y0 + r) * L + S.x0), o);
+        st4(F + S.off + r * S.rs, o);
       }
     }
-    copy_blk<R, BY>(Rv, Xn);
-    __syncthreads();  // the next slice reuses exchange buffers 0/1
   }
 }
 
@@ -772,91 +804,98 @@ static int prepare_smem(K kernel, size_t bytes) {
   return QEDF_OK;
 }
 
-static int max_threads_by(int by) {
-  return by == 2 ? MaxThreads<2>::value : (by == 4 ? MaxThreads<4>::value : MaxThreads<6>::value);
-}
-
 bool by_valid(int L, int by) {
   return (by == 2 || by == 4 || by == 6) && L % by == 0 && (L / 2) * (L / by) <= max_threads_by(by);
 }
 
+// slices of an operator kernel that one SM holds at a time, by the warps that
+// its registers allow (the launch bounds above)
+static int resident_slices(int L, int by, int real_bytes) {
+  const int warps = slice_threads(L, by) / 32;
+  const int room = real_bytes == 4 ? (by == 2 ? 36 : by == 4 ? 16 : 12) : (by == 2 ? 20 : warps > 12 ? 16 : 12);
+  return room / warps;
+}
+
+// The tile height that keeps most slices resident per SM; at equal numbers the
+// taller tile in single precision (less exchange per site: L = 36, 8 right-hand
+// sides, M^dag M 31 us with 2 x 6, 35 with 2 x 2 tiles; L = 30, 22.8 and 24.9),
+// the lower one in double, whose taller tiles spill (L = 48: 185 us with 2 x 2,
+// 209 with 2 x 4; where 2 x 4 fits two slices and 2 x 2 one, L = 36, 86 against
+// 95 us; 2 x 6 only where nothing else divides L: L = 30, 80 against 58 us,
+// L = 60, 149 against 142 us with 2 x 4).
 int pick_by(int L, int requested, int real_bytes) {
   if (requested > 0) return by_valid(L, requested) ? requested : -1;
-  // single precision: the smallest tile that fits; double precision keeps
-  // 2 x 2 tiles only for small slices (register budget of 576-thread blocks)
-  if (real_bytes == 4) {
-    const int cands[3] = {2, 4, 6};
-    for (int c : cands)
-      if (by_valid(L, c)) return c;
-  } else {
-    if (by_valid(L, 2) && (L / 2) * (L / 2) <= 256) return 2;
-    const int cands[3] = {4, 6, 2};
-    for (int c : cands)
-      if (by_valid(L, c)) return c;
+  int best = -1, most = 0;
+  for (int by : {2, 4, 6}) {
+    if (!by_valid(L, by) || (real_bytes == 8 && by == 6 && best > 0)) continue;
+    const int n = resident_slices(L, by, real_bytes);
+    if (best < 0 || n > most || (n == most && real_bytes == 4)) {
+      best = by;
+      most = n;
+    }
   }
-  return -1;
+  return best;
 }
 
 static size_t smem_limit() { return 227 * 1024; }
 
-template <typename R, typename A, int BY, int EC>
-static int launch_operator_t(int op, const OpArgs& a, cudaStream_t st) {
-  const int threads = slice_threads(a.L, BY, (EC & EC_XS) != 0);
-  const size_t smem = slice_smem_bytes<R, EC>(a.L, BY, 2);
-  if (smem > smem_limit() || threads > MaxT<BY, EC>::value) return QEDF_ERR_SIZE;
-  dim3 grid((a.Nt + a.T - 1) / a.T, a.bs);
-  if (op == OP_M) {
-    if (prepare_smem(k_operator<R, A, BY, OP_M, EC>, smem)) return QEDF_ERR_CUDA;
-    k_operator<R, A, BY, OP_M, EC><<<grid, threads, smem, st>>>(a);
-  } else if (op == OP_MH) {
-    if (prepare_smem(k_operator<R, A, BY, OP_MH, EC>, smem)) return QEDF_ERR_CUDA;
-    k_operator<R, A, BY, OP_MH, EC><<<grid, threads, smem, st>>>(a);
-  } else {
-    if (prepare_smem(k_operator<R, A, BY, OP_MHM, EC>, smem)) return QEDF_ERR_CUDA;
-    k_operator<R, A, BY, OP_MHM, EC><<<grid, threads, smem, st>>>(a);
+// blocks of a run-per-block kernel: as many as the GPU holds at once, but
+// with a slab length one per slab
+template <typename K>
+static int run_grid(K kernel, int threads, size_t smem, int bs, int Nt, int T, int& grid) {
+  if (prepare_smem(kernel, smem)) return QEDF_ERR_CUDA;
+  const int64_t W = (int64_t)bs * Nt;
+  int64_t g = (int64_t)bs * ((Nt + (T > 0 ? T : 1) - 1) / (T > 0 ? T : 1));
+  if (T <= 0 && W > num_sms()) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
+      return QEDF_ERR_SIZE;
+    g = std::min<int64_t>(W, (int64_t)num_sms() * per_sm);
   }
+  if (g > INT32_MAX) return QEDF_ERR_SIZE;
+  grid = (int)g;
+  return QEDF_OK;
+}
+
+template <typename R, typename A, int BY, int OP, int CFG>
+static int launch_operator_t(const OpArgs& a, cudaStream_t st) {
+  const int threads = slice_threads(a.L, BY);
+  constexpr int rec = Slice<R, BY, CFG == CFG_TALL, CFG == CFG_TALL ? 1 : 2>::REC;
+  const size_t smem =
+      slice_smem<R>(threads, rec) + (OP == OP_MHM && CFG == CFG_REG ? stash_smem<R, BY>(threads) : 0);
+  if (smem > smem_limit() || threads > OpT<R, BY, CFG>::threads) return QEDF_ERR_SIZE;
+  auto kern = k_operator<R, A, BY, OP, CFG>;
+  int grid = 0;
+  if (int e = run_grid(kern, threads, smem, a.bs, a.Nt, a.T, grid)) return e;
+  kern<<<grid, threads, smem, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
 }
 
-// Lattice sides with engines compiled for a fixed L (the benchmark lattice,
-// L = 48); every other L runs the run-time-L engine.
-template <typename R, typename A, int BY, int EC>
-static int launch_operator_fl(int op, const OpArgs& a, cudaStream_t st) {
-  if constexpr (EC == 0 || EC == EC_PHS)
-    return with_fixed_l<BY>(a.L, [&](auto lt) {
-      return launch_operator_t<R, A, BY, EC | EC_L(decltype(lt)::value)>(op, a, st);
-    });
-  return launch_operator_t<R, A, BY, EC>(op, a, st);
-}
-
-// double precision keeps the phases in shared memory when they fit; without
-// room for the stash, y stays in registers
 template <typename R, typename A, int BY>
-static int launch_operator_by(int op, const OpArgs& a, int xs, cudaStream_t st) {
-  if (sizeof(R) == 8 && slice_smem_bytes<R, EC_PHS>(a.L, BY, 2) <= smem_limit())
-    return launch_operator_fl<R, A, BY, EC_PHS>(op, a, st);
-  if (sizeof(R) == 4 && xs && xs_possible(a.L) && ((a.L / 2) & (a.L / 2 - 1)) == 0 &&
-      slice_threads(a.L, BY, true) <= MaxT<BY, EC_XS>::value)
-    return launch_operator_t<R, A, BY, EC_XS>(op, a, st);
-  if (slice_smem_bytes<R, 0>(a.L, BY, 2) <= smem_limit()) return launch_operator_fl<R, A, BY, 0>(op, a, st);
-  return launch_operator_t<R, A, BY, EC_NOSTASH>(op, a, st);
+static int launch_operator_by(int op, const OpArgs& a, cudaStream_t st) {
+  // double precision: 2 x 6 tiles and 2 x 4 tiles above 384 threads
+  if constexpr (sizeof(R) == 8 && BY >= 4) {
+    if (BY == 6 || slice_threads(a.L, BY) > OpT<R, BY, CFG_REG>::threads) {
+      if (op == OP_M) return launch_operator_t<R, A, BY, OP_M, CFG_TALL>(a, st);
+      if (op == OP_MH) return launch_operator_t<R, A, BY, OP_MH, CFG_TALL>(a, st);
+      return launch_operator_t<R, A, BY, OP_MHM, CFG_TALL>(a, st);
+    }
+  }
+  if constexpr (!(sizeof(R) == 8 && BY == 6)) {
+    if (op == OP_M) return launch_operator_t<R, A, BY, OP_M, CFG_REG>(a, st);
+    if (op == OP_MH) return launch_operator_t<R, A, BY, OP_MH, CFG_REG>(a, st);
+    return launch_operator_t<R, A, BY, OP_MHM, CFG_REG>(a, st);
+  }
+  return QEDF_ERR_ARG;
 }
 
 template <typename R, typename A>
 int launch_operator(int op, OpArgs a, int by, cudaStream_t st) {
   by = pick_by(a.L, by, sizeof(R));
-  if (by < 0) return QEDF_ERR_ARG;
-  if (a.T <= 0) {
-    // spread the slabs over about two waves of the SMs
-    const long want = 2L * num_sms();
-    long slabs = std::max(1L, want / std::max(1, a.bs));
-    a.T = (int)std::max(1L, (a.Nt + slabs - 1) / slabs);
-  }
-  const int xs = a.xs;
   switch (by) {
-    case 2: return launch_operator_by<R, A, 2>(op, a, xs, st);
-    case 4: return launch_operator_by<R, A, 4>(op, a, xs, st);
-    case 6: return launch_operator_by<R, A, 6>(op, a, xs, st);
+    case 2: return launch_operator_by<R, A, 2>(op, a, st);
+    case 4: return launch_operator_by<R, A, 4>(op, a, st);
+    case 6: return launch_operator_by<R, A, 6>(op, a, st);
   }
   return QEDF_ERR_ARG;
 }
@@ -865,11 +904,11 @@ template int launch_operator<double, double>(int, OpArgs, int, cudaStream_t);
 
 template <typename R, typename A, int BY>
 static int launch_bvec_by(const BvecArgs& a, int nvec, cudaStream_t st) {
-  const int threads = ((a.L / 2) * (a.L / BY) + 31) / 32 * 32;
-  const size_t smem = slice_smem_bytes<R, 0>(a.L, BY, 2);
+  const int threads = slice_threads(a.L, BY);
+  const size_t smem = slice_smem<R>(threads, Slice<R, BY>::REC);
   if (smem > smem_limit()) return QEDF_ERR_SIZE;
-  if (prepare_smem(k_bvec<R, A, BY, false>, smem)) return QEDF_ERR_CUDA;
-  k_bvec<R, A, BY, false><<<nvec, threads, smem, st>>>(a);
+  if (prepare_smem(k_bvec<R, A, BY>, smem)) return QEDF_ERR_CUDA;
+  k_bvec<R, A, BY><<<nvec, threads, smem, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
 }
 
@@ -915,35 +954,21 @@ int launch_precon(const PreconArgs& a, cudaStream_t st) {
 template int launch_precon<float>(const PreconArgs&, cudaStream_t);
 template int launch_precon<double>(const PreconArgs&, cudaStream_t);
 
-template <typename R, typename A, int BY, bool PHS, int LT = 0>
-static int launch_force_t(const ForceArgs& a, cudaStream_t st) {
-  const int threads = ((a.L / 2) * (a.L / BY) + 31) / 32 * 32;
-  // four exchange buffers; the force keeps no stash
-  const size_t smem = slice_smem_bytes<R, (PHS ? EC_PHS : 0) | EC_NOSTASH>(a.L, BY, 4);
-  if (smem > smem_limit()) return QEDF_ERR_SIZE;
-  if (prepare_smem(k_force<R, A, BY, PHS, LT>, smem)) return QEDF_ERR_CUDA;
-  dim3 grid((a.Nt + a.T - 1) / a.T, a.bs);
-  k_force<R, A, BY, PHS, LT><<<grid, threads, smem, st>>>(a);
-  return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
-}
-
 template <typename R, typename A, int BY>
 static int launch_force_by(const ForceArgs& a, cudaStream_t st) {
-  // the benchmark lattices run engines compiled for their size
-  if (sizeof(R) == 8 && slice_smem_bytes<R, EC_PHS | EC_NOSTASH>(a.L, BY, 4) <= smem_limit())
-    return with_fixed_l<BY>(a.L, [&](auto lt) { return launch_force_t<R, A, BY, true, decltype(lt)::value>(a, st); });
-  return with_fixed_l<BY>(a.L, [&](auto lt) { return launch_force_t<R, A, BY, false, decltype(lt)::value>(a, st); });
+  const int threads = slice_threads(a.L, BY);
+  const size_t smem = slice_smem<R>(threads, ForceSlice<R, BY>::REC);
+  if (smem > smem_limit() || threads > ForceT<R, BY>::threads) return QEDF_ERR_SIZE;
+  auto kern = k_force<R, A, BY>;
+  int grid = 0;
+  if (int e = run_grid(kern, threads, smem, a.bs, a.Nt, a.T, grid)) return e;
+  kern<<<grid, threads, smem, st>>>(a);
+  return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
 }
 
 template <typename R, typename A>
 int launch_force(ForceArgs a, int by, cudaStream_t st) {
   by = pick_by(a.L, by, sizeof(R));
-  if (by < 0) return QEDF_ERR_ARG;
-  if (a.T <= 0) {
-    const long want = 2L * num_sms();
-    long slabs = std::max(1L, want / std::max(1, a.bs));
-    a.T = (int)std::max(1L, (a.Nt + slabs - 1) / slabs);
-  }
   switch (by) {
     case 2: return launch_force_by<R, A, 2>(a, st);
     case 4: return launch_force_by<R, A, 4>(a, st);

@@ -43,7 +43,7 @@
 
 #include "qedf_internal.h"
 #include "qedf_precon_table.h"
-#include "qedf_slice.cuh"
+#include "qedf_slice_pcg.cuh"
 
 namespace qedf {
 

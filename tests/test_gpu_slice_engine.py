@@ -51,3 +51,38 @@ def test_mixed_solve_takes_the_double_solves_iterations(L, Nt):
         assert int(res.status.max()) == 0
         its[mode] = int(res.iters.max())
     assert its["mixed"] <= 1.2 * its["fp64"] + 10
+
+
+@pytest.mark.parametrize("prec", ["c64", "c128"])
+@pytest.mark.parametrize("L,Nt,bs", [(2, 5, 2000), (4, 7, 1500), (18, 5, 700), (28, 3, 301)])
+def test_runs_across_right_hand_sides_match_slabs(L, Nt, bs, prec):
+    """More slices than the GPU holds blocks: a block's run of slices ends one
+    right-hand side and begins the next.  The same arithmetic per slice as with
+    one slab per block, so the results are equal bit for bit."""
+    from qed_fermion_b200 import ops
+    cdt, rdt = (torch.complex64, torch.float32) if prec == "c64" else (torch.complex128, torch.float64)
+    g = torch.Generator(device=DEV).manual_seed(L)
+    phi = torch.randn((bs, 2 * L * L * Nt), device=DEV, dtype=rdt, generator=g)
+    x = torch.randn((bs, L * L * Nt), device=DEV, dtype=cdt, generator=g)
+    for op in ("m", "mh", "mhm"):
+        assert torch.equal(ops.apply_operator(op, phi, x, L, 0.1), ops.apply_operator(op, phi, x, L, 0.1, slab=Nt))
+    assert torch.equal(ops.fermion_force(phi, x, L, 0.1), ops.fermion_force(phi, x, L, 0.1, slab=2))
+
+
+@pytest.mark.parametrize("L,by", [(20, 2), (20, 4), (24, 2), (24, 4), (24, 6), (52, 4), (54, 6), (56, 4), (60, 4), (60, 6)])
+@pytest.mark.parametrize("prec,tol", [("c64", 1e-6), ("c128", 1e-13)])
+def test_tile_heights_match_oracle(L, by, prec, tol):
+    """Every tile height that a side allows, the operators and the force."""
+    from qed_fermion_b200 import ops
+    phi, v = _case(L, 5, 2, seed=L + by)
+    w = v.reshape(2, 5, L * L)
+    cdt, rdt = (torch.complex64, torch.float32) if prec == "c64" else (torch.complex128, torch.float64)
+    p, x = torch.tensor(phi.reshape(2, -1), dtype=rdt, device=DEV), torch.tensor(v, dtype=cdt, device=DEV)
+    for op, f in (("m", O.m_vec), ("mh", O.mh_vec), ("mhm", O.mhm_vec)):
+        want = f(phi, w, L, 0.1).reshape(2, -1)
+        got = ops.apply_operator(op, p, x, L, 0.1, by=by).cpu().numpy()
+        assert np.abs(got - want).max() < tol * np.abs(want).max()
+    want = O.force_f_from_xi(phi, w, L, 0.1).reshape(2, -1)
+    got = ops.fermion_force(p, x, L, 0.1, by=by).cpu().numpy()
+    # the force's tolerances of the parity tests
+    assert np.abs(got - want).max() < (2e-5 if prec == "c64" else 1e-12) * np.abs(want).max()
