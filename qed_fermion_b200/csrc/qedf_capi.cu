@@ -104,12 +104,10 @@ int force_entry(const R* boson, const R* xi, R* F, int bs, int Lx, int Ltau, dou
   a.bs = bs;
   a.rhs_per_phi = rhs_per_boson;
   a.T = slab;
+  a.c1 = f.c1;
+  a.ch = f.ch;
   a.t1 = f.t1;
   a.th = f.th;
-  a.Cb = f.Cb;
-  const double c[7] = {f.ch, f.ch, f.ch, f.c1, f.ch, f.ch, f.ch};
-  double k = 2 * f.Cb;
-  for (int i = 0; i < 7; ++i) a.kappa[i] = (k *= c[i] * c[i]);
   return launch_force<R, R>(a, by, reinterpret_cast<cudaStream_t>(stream));
 }
 

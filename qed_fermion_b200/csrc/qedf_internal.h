@@ -42,8 +42,7 @@ struct ForceArgs {
   const void* xi;
   void* F;
   int L, Nt, bs, rhs_per_phi, T;
-  double t1, th, Cb;
-  double kappa[7];  // scalars of the force terms at the seven factor positions (k_force)
+  double c1, ch, t1, th;
 };
 
 struct BosonArgs {

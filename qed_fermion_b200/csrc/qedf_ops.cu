@@ -379,43 +379,111 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_precon_band(Pre
 // sum that the reference evaluates with explicit partial products
 // (force_f_fast, hmc_sampler_batch.py:2150-2227; force_f_sparse :2230-2330).
 //
-// The factors are applied without their scalars c_j, backwards as I - tK
-// ((I - tK)(I + tK) = I / c^2), so at position k the bond terms carry
-// kappa_k = 2 Cb prod_{j<=k} c_j^2.  The exchange is the engine's: a cross bond's owner
-// exports conj(a) R_i and conj(a) l_i and gets R_j and l_j, which is all that
-// its own force term and both updates need.  Every slice is independent of
-// the others: the slices of all right-hand sides are dealt as block_run does.
-// Measured, 2 right-hand sides at L = 48, Ltau = 480, complex64:
-// 31 us, against 39 with fixed slabs and an engine that exchanged both vectors and phases.
+// Unlike the operators, the force exchanges plain values and its bonds' phases
+// (once per slice, in the record's last entries) and applies the factors with
+// their scalars: every rounding is then that of the textbook update of each
+// site, so that trajectories in single precision, whose energies show a change
+// of the last bit of the force at 1e-9, do not depend on the tiling.  Every
+// slice is independent of the others: the slices of all right-hand sides are
+// dealt as block_run does.  Measured, 2 right-hand sides at L = 48, Ltau = 480,
+// complex64: 35 us, against 39 with fixed slabs and one block per SM.
 template <typename R, int BY>
 struct ForceT {
   static constexpr int threads = MaxT<R, BY>::value;
 };
 
 template <typename R, int BY>
-struct ForceSlice : Slice<R, BY, false, 2, 2> {
-  using Base = Slice<R, BY, false, 2, 2>;
+struct ForceSlice : Slice<R, BY, false, 2, 2, BY + 2> {
+  using Base = Slice<R, BY, false, 2, 2, BY + 2>;
+  static constexpr int PHX = Base::PH0, PHY = PHX + BY;  // x-bond phases of column x0+1, y-bond ones of the last row
+  R c1, ch;
 
-  // kappa-free term of one bond, R after the factor's inverse, l before it:
-  // Re[conj(l_i) (i a) R_j + conj(l_j) conj(i a) R_i]
-  __device__ static __forceinline__ R term(Cx<R> li, Cx<R> lj, Cx<R> Ri, Cx<R> Rj, Cx<R> a) {
-    // X = conj(l_i) R_j, Y = conj(l_j) R_i
-    const R d1 = fma(lj.re, Ri.im, fma(-lj.im, Ri.re, fma(-li.re, Rj.im, li.im * Rj.re)));  // Im Y - Im X
-    const R d2 = fma(lj.re, Ri.re, fma(lj.im, Ri.im, fma(li.re, Rj.re, li.im * Rj.im)));    // Re X + Re Y
-    return fma(a.re, d1, -(a.im * d2));
+  // makes the phases that the neighbours need visible at the next barrier
+  __device__ __forceinline__ void publish() {
+#pragma unroll
+    for (int r = 0; r < BY; ++r) this->me[PHX + r] = this->px(r, 1);
+    this->me[PHY] = this->py(BY - 1, 0);
+    this->me[PHY + 1] = this->py(BY - 1, 1);
+  }
+  // v_i + a v_j and v_j + conj(a) v_i, times c
+  __device__ static __forceinline__ Cx<R> upd(R c, Cx<R> a, Cx<R> vj, Cx<R> vi) { return c * cfma(a, vj, vi); }
+  __device__ static __forceinline__ Cx<R> updj(R c, Cx<R> a, Cx<R> vi, Cx<R> vj) { return c * cjfma(a, vi, vj); }
+
+  // v <- F_g v, plain values exchanged
+  template <int G, int BUF>
+  __device__ __forceinline__ void factor_true(Cx<R> (&v)[BY][2]) {
+    constexpr int B0 = BUF * 2 * BY;
+    const R c = G == 0 ? c1 : ch;
+    Cx<R>* me = this->me;
+    auto local = [&](Cx<R>& vi, Cx<R>& vj, Cx<R> a) {
+      const Cx<R> oi = vi, oj = vj;
+      vi = upd(c, a, oj, oi);
+      vj = updj(c, a, oi, oj);
+    };
+    if constexpr (G == 0 || G == 2) {
+      constexpr int RC = G == 0 ? 1 : 0;
+#pragma unroll
+      for (int r = RC; r < BY; r += 2) {
+        me[B0 + (r & ~1)] = v[r][0];
+        me[B0 + (r & ~1) + 1] = v[r][1];
+      }
+#pragma unroll
+      for (int r = 1 - RC; r < BY; r += 2) local(v[r][0], v[r][1], this->px(r, 0));
+      __syncthreads();
+#pragma unroll
+      for (int r = RC; r < BY; r += 2) {
+        v[r][1] = upd(c, this->px(r, 1), this->rt[B0 + (r & ~1)], v[r][1]);
+        v[r][0] = updj(c, this->lf[PHX + r], this->lf[B0 + (r & ~1) + 1], v[r][0]);
+      }
+    } else {
+      constexpr int CL = (G == 1) ? 0 : 1, CC = 1 - CL;
+      me[B0] = v[0][CC];
+      me[B0 + 1] = v[BY - 1][CC];
+#pragma unroll
+      for (int r = 0; r < BY; r += 2) local(v[r][CL], v[r + 1][CL], this->py(r, CL));
+#pragma unroll
+      for (int r = 1; r + 1 < BY; r += 2) local(v[r][CC], v[r + 1][CC], this->py(r, CC));
+      __syncthreads();
+      v[BY - 1][CC] = upd(c, this->py(BY - 1, CC), this->dn[B0], v[BY - 1][CC]);
+      v[0][CC] = updj(c, this->up[PHY + CC], this->up[B0 + 1], v[0][CC]);
+    }
+  }
+
+  // term for one bond: 2 c Re[conj(l_i) (i a) R_j + conj(l_j) conj(i a) R_i]
+  __device__ static __forceinline__ R term(Cx<R> li, Cx<R> lj, Cx<R> Ri, Cx<R> Rj, Cx<R> a, R c) {
+    const Cx<R> ia = mk<R>(-a.im, a.re);
+    const Cx<R> u = cjmul(li, cmul(ia, Rj));
+    const Cx<R> w = cjmul(lj, cjmul(ia, Ri));
+    return (R)2 * c * (u.re + w.re);
   }
   // a bond inside the tile
-  __device__ static __forceinline__ void local(Cx<R>& Ri, Cx<R>& Rj, Cx<R>& li, Cx<R>& lj, Cx<R> a, R kap, R& F) {
-    Base::pair(Ri, Rj, mk<R>(-a.re, -a.im));
-    F = fma(kap, term(li, lj, Ri, Rj, a), F);
-    Base::pair(li, lj, a);
+  __device__ static __forceinline__ void local(Cx<R>& Ri, Cx<R>& Rj, Cx<R>& li, Cx<R>& lj, Cx<R> a, R c, R& F) {
+    const Cx<R> nRi = upd(c, cneg(a), Rj, Ri), nRj = updj(c, cneg(a), Ri, Rj);
+    F += term(li, lj, nRi, nRj, a, c);
+    const Cx<R> oi = li, oj = lj;
+    li = upd(c, a, oj, oi);
+    lj = updj(c, a, oi, oj);
+    Ri = nRi;
+    Rj = nRj;
+  }
+  // the owner's side of a cross bond: i is its own site, j the neighbour's
+  __device__ static __forceinline__ void edge(Cx<R>& Ri, Cx<R>& li, Cx<R> Rj, Cx<R> lj, Cx<R> a, R c, R& F) {
+    const Cx<R> nRi = upd(c, cneg(a), Rj, Ri), nRj = updj(c, cneg(a), Ri, Rj);
+    F += term(li, lj, nRi, nRj, a, c);
+    li = upd(c, a, lj, li);
+    Ri = nRi;
+  }
+  // the other side: j is its own site
+  __device__ static __forceinline__ void far(Cx<R>& Rj, Cx<R>& lj, Cx<R> Ri, Cx<R> li, Cx<R> a, R c) {
+    Rj = updj(c, cneg(a), Ri, Rj);
+    lj = updj(c, a, li, lj);
   }
 
-  // one factor position: R <- (I - K_g) R, accumulate the force, l <- (I + K_g) l
+  // one factor position: R <- F_g^{-1} R, accumulate the force, l <- F_g l
   template <int G, int BUF>
-  __device__ __forceinline__ void step(Cx<R> (&Rv)[BY][2], Cx<R> (&l)[BY][2], R (&Fx)[BY][2], R (&Fy)[BY][2],
-                                       R kap) {
+  __device__ __forceinline__ void step(Cx<R> (&Rv)[BY][2], Cx<R> (&l)[BY][2], R (&Fx)[BY][2], R (&Fy)[BY][2]) {
     constexpr int B0 = BUF * 2 * BY, B1 = B0 + BY;  // exchange slots of R and l
+    const R c = G == 0 ? c1 : ch;
     Cx<R>* me = this->me;
     if constexpr (G == 0 || G == 2) {
       constexpr int RC = G == 0 ? 1 : 0;
@@ -423,47 +491,36 @@ struct ForceSlice : Slice<R, BY, false, 2, 2> {
       for (int r = RC; r < BY; r += 2) {
         const int q = r & ~1;
         me[B0 + q] = Rv[r][0];
-        me[B0 + q + 1] = Base::cjm(this->px(r, 1), Rv[r][1]);
+        me[B0 + q + 1] = Rv[r][1];
         me[B1 + q] = l[r][0];
-        me[B1 + q + 1] = Base::cjm(this->px(r, 1), l[r][1]);
+        me[B1 + q + 1] = l[r][1];
       }
 #pragma unroll
       for (int r = 1 - RC; r < BY; r += 2)
-        local(Rv[r][0], Rv[r][1], l[r][0], l[r][1], this->px(r, 0), kap, Fx[r][0]);
+        local(Rv[r][0], Rv[r][1], l[r][0], l[r][1], this->px(r, 0), c, Fx[r][0]);
       __syncthreads();
 #pragma unroll
       for (int r = RC; r < BY; r += 2) {
         const int q = r & ~1;
-        const Cx<R> a = this->px(r, 1);
-        edge(Rv[r][1], l[r][1], this->rt[B0 + q], this->rt[B1 + q], a, kap, Fx[r][1]);
-        Rv[r][0] = Rv[r][0] - this->lf[B0 + q + 1];
-        l[r][0] = l[r][0] + this->lf[B1 + q + 1];
+        edge(Rv[r][1], l[r][1], this->rt[B0 + q], this->rt[B1 + q], this->px(r, 1), c, Fx[r][1]);
+        far(Rv[r][0], l[r][0], this->lf[B0 + q + 1], this->lf[B1 + q + 1], this->lf[PHX + r], c);
       }
     } else {
       constexpr int CL = (G == 1) ? 0 : 1, CC = 1 - CL;
-      const Cx<R> a = this->py(BY - 1, CC);
       me[B0] = Rv[0][CC];
-      me[B0 + 1] = Base::cjm(a, Rv[BY - 1][CC]);
+      me[B0 + 1] = Rv[BY - 1][CC];
       me[B1] = l[0][CC];
-      me[B1 + 1] = Base::cjm(a, l[BY - 1][CC]);
+      me[B1 + 1] = l[BY - 1][CC];
 #pragma unroll
       for (int r = 0; r < BY; r += 2)
-        local(Rv[r][CL], Rv[r + 1][CL], l[r][CL], l[r + 1][CL], this->py(r, CL), kap, Fy[r][CL]);
+        local(Rv[r][CL], Rv[r + 1][CL], l[r][CL], l[r + 1][CL], this->py(r, CL), c, Fy[r][CL]);
 #pragma unroll
       for (int r = 1; r + 1 < BY; r += 2)
-        local(Rv[r][CC], Rv[r + 1][CC], l[r][CC], l[r + 1][CC], this->py(r, CC), kap, Fy[r][CC]);
+        local(Rv[r][CC], Rv[r + 1][CC], l[r][CC], l[r + 1][CC], this->py(r, CC), c, Fy[r][CC]);
       __syncthreads();
-      edge(Rv[BY - 1][CC], l[BY - 1][CC], this->dn[B0], this->dn[B1], a, kap, Fy[BY - 1][CC]);
-      Rv[0][CC] = Rv[0][CC] - this->up[B0 + 1];
-      l[0][CC] = l[0][CC] + this->up[B1 + 1];
+      edge(Rv[BY - 1][CC], l[BY - 1][CC], this->dn[B0], this->dn[B1], this->py(BY - 1, CC), c, Fy[BY - 1][CC]);
+      far(Rv[0][CC], l[0][CC], this->up[B0 + 1], this->up[B1 + 1], this->up[PHY + CC], c);
     }
-  }
-  // the owner's side of a cross bond: i is its own site, j the neighbour's
-  __device__ static __forceinline__ void edge(Cx<R>& Ri, Cx<R>& li, Cx<R> Rj, Cx<R> lj, Cx<R> a, R kap, R& F) {
-    Cx<R> nj = Rj;
-    Base::pair(Ri, nj, mk<R>(-a.re, -a.im));
-    F = fma(kap, term(li, lj, Ri, nj, a), F);
-    li = cfma(a, lj, li);
   }
 };
 
@@ -474,10 +531,9 @@ __global__ void __launch_bounds__(ForceT<R, BY>::threads, 1) k_force(ForceArgs p
   S.init(p.L, smem, threadIdx.x);
   const size_t sv = 2 * (size_t)p.L * p.L;
   const int Nt = p.Nt;
-  const R t1 = (R)p.t1, th = (R)p.th, Cb = (R)p.Cb;
-  R kap[7];
-#pragma unroll
-  for (int k = 0; k < 7; ++k) kap[k] = (R)p.kappa[k];
+  const R t1 = (R)p.t1, th = (R)p.th;
+  S.c1 = (R)p.c1;
+  S.ch = (R)p.ch;
   int64_t w, w1;
   block_run(p.bs, Nt, p.T, w, w1);
   for (; w < w1; ++w) {
@@ -489,30 +545,26 @@ __global__ void __launch_bounds__(ForceT<R, BY>::threads, 1) k_force(ForceArgs p
     S.load(Rv, xi + t * sv);
     S.phases_of(phi + t * sv, t1, th);
     S.load(l, xi + tn * sv);
-    S.template factor<3, 0>(Rv);  // R_7 = B_t xi_t
-    S.template factor<2, 1>(Rv);
-    S.template factor<1, 0>(Rv);
-    S.template factor<0, 1>(Rv);
-    S.template factor<1, 0>(Rv);
-    S.template factor<2, 1>(Rv);
-    S.template factor<3, 0>(Rv);
-    const R sg = sigma_of<R>(t, Nt);
+    S.publish();
+    S.template factor_true<3, 0>(Rv);  // R_7 = B_t xi_t
+    S.template factor_true<2, 1>(Rv);
+    S.template factor_true<1, 0>(Rv);
+    S.template factor_true<0, 1>(Rv);
+    S.template factor_true<1, 0>(Rv);
+    S.template factor_true<2, 1>(Rv);
+    S.template factor_true<3, 0>(Rv);
+    axpy_blk<R, BY>(l, Rv, sigma_of<R>(t, Nt), l);
     R Fx[BY][2], Fy[BY][2];
 #pragma unroll
-    for (int r = 0; r < BY; ++r)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        l[r][c] = mk<R>(fma(Cb, Rv[r][c].re, -sg * l[r][c].re), fma(Cb, Rv[r][c].im, -sg * l[r][c].im));
-        Fx[r][c] = Fy[r][c] = 0;
-      }
+    for (int r = 0; r < BY; ++r) Fx[r][0] = Fx[r][1] = Fy[r][0] = Fy[r][1] = 0;
     // positions k = 1..7 of B = F4 F3 F2 F1 F2 F3 F4
-    S.template step<3, 1>(Rv, l, Fx, Fy, kap[0]);
-    S.template step<2, 0>(Rv, l, Fx, Fy, kap[1]);
-    S.template step<1, 1>(Rv, l, Fx, Fy, kap[2]);
-    S.template step<0, 0>(Rv, l, Fx, Fy, kap[3]);
-    S.template step<1, 1>(Rv, l, Fx, Fy, kap[4]);
-    S.template step<2, 0>(Rv, l, Fx, Fy, kap[5]);
-    S.template step<3, 1>(Rv, l, Fx, Fy, kap[6]);
+    S.template step<3, 1>(Rv, l, Fx, Fy);
+    S.template step<2, 0>(Rv, l, Fx, Fy);
+    S.template step<1, 1>(Rv, l, Fx, Fy);
+    S.template step<0, 0>(Rv, l, Fx, Fy);
+    S.template step<1, 1>(Rv, l, Fx, Fy);
+    S.template step<2, 0>(Rv, l, Fx, Fy);
+    S.template step<3, 1>(Rv, l, Fx, Fy);
     if (S.on) {
 #pragma unroll
       for (int r = 0; r < BY; ++r) {
@@ -520,6 +572,7 @@ __global__ void __launch_bounds__(ForceT<R, BY>::threads, 1) k_force(ForceArgs p
         st4(F + S.off + r * S.rs, o);
       }
     }
+    __syncthreads();  // the phases of this slice are read
   }
 }
 

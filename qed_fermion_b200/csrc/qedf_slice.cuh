@@ -66,8 +66,8 @@ __host__ __device__ inline int slice_threads(int L, int BY) { return ((L / 2) * 
 
 // complex entries of a thread's record: nbuf exchange buffers of `vecs`
 // vectors, BY slots each, and with phs its 4 BY bond phases; odd
-__host__ __device__ constexpr int slice_record(int BY, int nbuf, int vecs, bool phs) {
-  return (nbuf * vecs * BY + (phs ? 4 * BY : 0)) | 1;
+__host__ __device__ constexpr int slice_record(int BY, int nbuf, int vecs, bool phs, int extra) {
+  return (nbuf * vecs * BY + (phs ? 4 * BY : 0) + extra) | 1;
 }
 // complex entries of a thread's stash of one tile (16-byte units an odd number apart)
 template <typename R, int BY>
@@ -96,13 +96,17 @@ struct Stash {
 // NBUF exchange buffers of VECS vectors per thread.  NBUF = 1 (a second
 // barrier per factor instead of a second buffer) is for kernels short of
 // shared memory.
-template <typename R, int BY, bool PHS = false, int NBUF = 2, int VECS = 1>
+// A block may have more threads than its engine: init_named's barriers count the
+// engine's threads alone (whole warps).
+// EXTRA: further entries of the record, the kernel's own.
+template <typename R, int BY, bool PHS = false, int NBUF = 2, int VECS = 1, int EXTRA = 0>
 struct Slice {
   static_assert(BY % 2 == 0, "BY must be even");
-  static constexpr int REC = slice_record(BY, NBUF, VECS, PHS);
-  static constexpr int PH0 = NBUF * VECS * BY;  // first phase of a record
+  static constexpr int REC = slice_record(BY, NBUF, VECS, PHS, EXTRA);
+  static constexpr int PH0 = NBUF * VECS * BY;  // first phase (or extra entry) of a record
   int off, rs;  // reals: this tile's first site in a slice, one row
   bool on;      // owns a tile
+  int nthr;     // threads at the engine's barriers; 0: the whole block
   Cx<R>*me, *lf, *rt, *up, *dn;  // records: own and the four neighbours'
   Cx<R> px_[PHS ? 1 : BY][2], py_[PHS ? 1 : BY][2];
 
@@ -120,6 +124,15 @@ struct Slice {
     rt = base + (on ? by * nbx + (bx + 1 == nbx ? 0 : bx + 1) : tid) * REC;
     up = base + (on ? (by == 0 ? nby - 1 : by - 1) * nbx + bx : tid) * REC;
     dn = base + (on ? (by + 1 == nby ? 0 : by + 1) * nbx + bx : tid) * REC;
+    nthr = 0;
+  }
+  __device__ __forceinline__ void init_named(int L, unsigned char* smem, int tid, int threads) {
+    init(L, smem, tid);
+    nthr = threads;
+  }
+  __device__ __forceinline__ void sync() const {
+    if (nthr) asm volatile("bar.sync 1, %0;\n" ::"r"(nthr) : "memory");
+    else __syncthreads();
   }
 
   // phase of the x-bond / y-bond starting at own site (x0+c, y0+r)
@@ -229,7 +242,7 @@ struct Slice {
   template <int G, int BUF>
   __device__ __forceinline__ void factor(Cx<R> (&v)[BY][2]) {
     constexpr int B0 = (NBUF == 2 ? BUF : 0) * BY;
-    if constexpr (NBUF == 1) __syncthreads();  // the last factor's values are read
+    if constexpr (NBUF == 1) sync();  // the last factor's values are read
     if constexpr (G == 0 || G == 2) {
       constexpr int RC = G == 0 ? 1 : 0;  // parity of the cross rows
 #pragma unroll
@@ -239,7 +252,7 @@ struct Slice {
       }
 #pragma unroll
       for (int r = 1 - RC; r < BY; r += 2) pair(v[r][0], v[r][1], px(r, 0));
-      __syncthreads();
+      sync();
 #pragma unroll
       for (int r = RC; r < BY; r += 2) {
         v[r][1] = cfma(px(r, 1), rt[B0 + (r & ~1)], v[r][1]);
@@ -254,7 +267,7 @@ struct Slice {
       for (int r = 0; r < BY; r += 2) pair(v[r][CL], v[r + 1][CL], py(r, CL));
 #pragma unroll
       for (int r = 1; r + 1 < BY; r += 2) pair(v[r][CC], v[r + 1][CC], py(r, CC));
-      __syncthreads();
+      sync();
       v[BY - 1][CC] = cfma(py(BY - 1, CC), dn[B0], v[BY - 1][CC]);
       v[0][CC] = v[0][CC] + up[B0 + 1];
     }
