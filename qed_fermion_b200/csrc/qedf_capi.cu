@@ -206,7 +206,7 @@ int pcg_solve_ws(const qedf_system* sys, int nsys, const void* boson, const void
 
 extern "C" {
 
-const char* qedf_version(void) { return "qedf 0.1.0 (sm_100a)"; }
+const char* qedf_version(void) { return "qedf 0.2.0 (sm_100a)"; }
 
 const char* qedf_status_string(int s) {
   switch (s) {

@@ -227,6 +227,28 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
+}
+// the same with an L2 policy: evict first, for data not read again before much
+// else has passed through L2
+__device__ __forceinline__ unsigned long long evict_first_policy() {
+  unsigned long long p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, unsigned long long policy) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void st2_first(float* p, Cx<float> a, Cx<float> b) {
+  __stcs(reinterpret_cast<float4*>(p), make_float4(a.re, a.im, b.re, b.im));
+}
+__device__ __forceinline__ void st2_first(double* p, Cx<double> a, Cx<double> b) {
+  __stcs(reinterpret_cast<double2*>(p), make_double2(a.re, a.im));
+  __stcs(reinterpret_cast<double2*>(p) + 1, make_double2(b.re, b.im));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }

@@ -89,14 +89,17 @@ int launch_cdot(const R* u, const R* v, int64_t n, int rows, double* out, cudaSt
 // ---- persistent PCG -------------------------------------------------------
 constexpr int PCG_MAX_SYS = 32;
 constexpr int PCG_MAX_RHS = 256;
-constexpr int PCG_CHUNK = 16;  // sites per elementwise unit where 32 does not fit (a multiple of 2)
+constexpr int PCG_CHUNK = 16;  // sites per elementwise unit (a multiple of 2)
+// blocks of the solver per SM at most: enough to overlap barriers and loads; more only
+// lengthen the grid barriers
+constexpr int PCG_MAX_PER_SM = 4;
 
 struct PcgSys {
   int L, Nt, nrhs, shared;
-  int T, nslab;          // operator slabs per rhs
+  int T, nslab;          // slices per operator unit, operator units per rhs
   int nchunk;            // site chunks per rhs (elementwise phases)
+  int seg, nseg;         // slices per elementwise unit, tau segments per rhs
   int rhs0;              // first global rhs index
-  int unitA0, unitE0;    // first operator / elementwise unit
   int64_t vec0;          // first complex element of the system in the packed vectors
   int64_t phi0;          // first real of the system in the packed angles
   int precon;
@@ -105,14 +108,13 @@ struct PcgSys {
 };
 
 struct PcgParams {
-  int nsys, nrhs, unitsA, unitsE, CH;
+  int nsys, nrhs, CH;
+  int eng_threads;  // threads of a block that the slice engine uses
   PcgSys sys[PCG_MAX_SYS];
   int mode;  // QEDF_PCG_PLAIN_F32, QEDF_PCG_PLAIN_F64, QEDF_PCG_MIXED, QEDF_PCG_MIXED_BF16, QEDF_PCG_MIXED_F16
-  int xs;    // allow the warp-shuffle engine for the single-precision iterations
-  int stage; // 1: allow the staged operator engine (EC_STAGE) where its shared memory fits
-  int stage_off;  // bytes: start of the operator passes' slice stages in dynamic shared memory
   int x_init;     // 1: x holds an initial guess on entry (the solve starts from b - A x)
   int l2;    // 0: L2 persisting window over the iteration vectors when they fit; -1: off
+  int split;  // 1: some system's elementwise units are tau segments (r is double-buffered)
   int max_iter, ru_interval;
   double rtol, ru_delta;
   double c1, ch, t1, th, Cb;
@@ -124,11 +126,13 @@ struct PcgParams {
   void* x;           // solution (same type as b)
   // workspace (sloppy precision vectors, each nvec_total complex)
   void* r;
+  void* r2;          // second buffer of r, or null
   void* p0;
   void* p1;
   void* z;
   void* Op;
   void* xlo;         // mixed only
+  void* y0;          // mixed only: half of the reliable updates' M x (the other half in Op)
   double* acc;       // accumulators
   float* ptab;       // periodic 13-band tau tables of the preconditioner, per system
   unsigned int* bar; // [0] count, [1] generation, [2] error
@@ -139,6 +143,12 @@ struct PcgParams {
   int ptab_len;        // floats of all preconditioner tables
   long long* prof;     // optional [8] cycle counters of block 0 (see k_pcg), or null
 };
+constexpr int PCG_ACC_PER_RHS = 11;
+
+// bytes that a whole tau column of an elementwise unit may have (the limit on Ltau)
+inline size_t pcg_column_limit(int real_bytes, int threads) {
+  return (size_t)227 * 1024 - 19 * 1024 - (real_bytes == 4 ? 128 * (size_t)threads : 0);
+}
 
 size_t pcg_workspace_bytes(const PcgParams& p, int sloppy_bytes);
 size_t pcg_carve(PcgParams& p, int sloppy_bytes, void* workspace, size_t* zero_bytes);
