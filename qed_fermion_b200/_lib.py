@@ -128,18 +128,21 @@ def load():
     return _LIB
 
 
+# launches that one call of an entry point stands for: qedf_pcg_solve launches a
+# small preparation kernel, the solver and, unless l2_persist is -1, the kernel
+# that releases the L2 window
+_PER_CALL = {n: (0 if n in _HOST_ONLY else 1) for n in SIGNATURES}
+
+
 def call(name, *args):
     """Call entry point ``name`` and raise ``QedfError`` on a non-zero status."""
-    lib = load()
-    st = getattr(lib, name)(*args)
-    if name not in _HOST_ONLY:
-        # qedf_pcg_solve launches a small preparation kernel, the solver and,
-        # unless l2_persist is -1, the kernel that releases the L2 window
-        if name.startswith("qedf_pcg_solve"):
-            opts = next((a for a in args if isinstance(a, QedfPcgOpts)), None)
-            LAUNCHES["count"] += 2 if (opts is not None and opts.l2_persist < 0) else 3
-        else:
-            LAUNCHES["count"] += 1
+    lib = _LIB or load()
+    st = lib.__dict__[name](*args)
+    if name.startswith("qedf_pcg_solve"):
+        opts = next((a for a in args if isinstance(a, QedfPcgOpts)), None)
+        LAUNCHES["count"] += 2 if (opts is not None and opts.l2_persist < 0) else 3
+    else:
+        LAUNCHES["count"] += _PER_CALL[name]
     if st != QEDF_OK:
         raise QedfError(name, st, lib.qedf_status_string(st).decode())
     return st

@@ -1,5 +1,6 @@
 // extern "C" entry points declared in include/qedf.h: argument validation on
 // the host, then the kernel launchers of qedf_ops.cu / qedf_pcg.cu.
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -168,6 +169,24 @@ int kick_entry(A* p, const A* F, A* x, const double* dt, const float* mask, doub
 
 namespace qedf {
 
+// The current device's SM clock rate.  The query takes 1 to 9 ms of host time on
+// B200, more than a whole solve of a small lattice, so each device's answer, a
+// constant, is asked for once.
+static int sm_clock_khz() {
+  static std::atomic<int> known[64];
+  int dev = 0, khz = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 2000000;
+  khz = known[dev].load(std::memory_order_relaxed);
+  if (khz <= 0) {
+    if (cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, dev) != cudaSuccess || khz <= 0) {
+      cudaGetLastError();
+      khz = 2000000;
+    }
+    known[dev].store(khz, std::memory_order_relaxed);
+  }
+  return khz;
+}
+
 // Solve with a caller-provided workspace (shared by qedf_pcg_solve and the
 // static-scratch entry point).
 int pcg_solve_ws(const qedf_system* sys, int nsys, const void* boson, const void* b, void* x, int* iters,
@@ -191,11 +210,7 @@ int pcg_solve_ws(const qedf_system* sys, int nsys, const void* boson, const void
   p.status = status;
   p.prof = opts->profile;
   const double tmo = opts->timeout_ms > 0 ? opts->timeout_ms : 2000.0;
-  int dev = 0, clk_khz = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&clk_khz, cudaDevAttrClockRate, dev);
-  if (clk_khz <= 0) clk_khz = 2000000;
-  p.timeout_cycles = (long long)(tmo * (double)clk_khz);
+  p.timeout_cycles = (long long)(tmo * (double)sm_clock_khz());
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // accumulators and barrier state start at zero; preconditioner tables
   if (int e2 = launch_pcg_prep(p, (int)(zero_bytes / 4), st)) return e2;
