@@ -79,7 +79,6 @@ int precon_entry(const R* r, R* out, int bs, int Lx, int Ltau, const int* row_pt
   a.L = Lx;
   a.Nt = Ltau;
   a.bs = bs;
-  a.TC = 16;
   a.row_ptr = row_ptr;
   a.col = col;
   a.val = val;

@@ -31,7 +31,7 @@ struct BvecArgs {
 struct PreconArgs {
   const void* r;
   void* z;
-  int L, Nt, bs, TC;
+  int L, Nt, bs;
   const int* row_ptr;  // tau-space CSR of P_tau (device)
   const int* col;
   const double* val;

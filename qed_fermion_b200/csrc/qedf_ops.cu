@@ -217,151 +217,150 @@ __global__ void __launch_bounds__(MaxT<R, BY>::value, 1) k_bvec(BvecArgs p) {
 // ============================================================================
 // preconditioner z = (P_tau (x) I) r, P_tau given as a tau-space CSR matrix
 // ============================================================================
+//
+// A warp forms C consecutive output rows of 32 sites; a block's warps take
+// neighbouring segments of tau, whose common rows meet in L1.  The C + 2H rows
+// of r that a banded P_tau needs are all loaded at once, into registers, while
+// the warp finds out which rows of its segment are the middle CSR row (t =
+// Ltau/2) shifted along tau - taps t-H .. t+H with the same values, as in the
+// bulk.  Those rows then need registers only, with the taps as constants.  The
+// others, a few at the ends of tau, are dealt to all warps of the block, which
+// run over the CSR row: a lane holds an entry, the warp reads eight rows of r
+// at a time.  Both orders of summation are the CSR order, so the two forms
+// agree bit for bit.  What is left is loads in flight against the 60 MB of the
+// first size below.  Measured against columns staged in shared memory: 8
+// vectors at L = 36, Ltau = 359, complex64, 29.5 -> 21 us (complex128 52 -> 37);
+// 8 at 48 / 480, 54 -> 43 us.  With the rows of r asked for before the entries,
+// 26 us: a load that depends on another one waits for both behind the queue.
+// Four warps to a block: with eight, 25 us, the blocks' last wave being emptier.
 template <typename R>
-__global__ void k_precon(PreconArgs p) {
-  const int Vs = p.L * p.L;
-  const int s = (blockIdx.x * blockDim.x + threadIdx.x) * 2;  // two sites per thread
-  if (s >= Vs) return;
-  const int rb = blockIdx.z;
-  const size_t sv = 2 * (size_t)Vs;
-  const R* r = reinterpret_cast<const R*>(p.r) + (size_t)rb * p.Nt * sv;
-  R* z = reinterpret_cast<R*>(p.z) + (size_t)rb * p.Nt * sv;
-  const int t0 = blockIdx.y * p.TC;
-  const int t1 = min(t0 + p.TC, p.Nt);
-  for (int t = t0; t < t1; ++t) {
-    Cx<R> acc0 = mk<R>(0, 0), acc1 = mk<R>(0, 0);
-    for (int k = p.row_ptr[t]; k < p.row_ptr[t + 1]; ++k) {
-      const R w = (R)p.val[k];
-      if ((unsigned)p.col[k] >= (unsigned)p.Nt) continue;  // outside the matrix
-      Cx<R> a, b;
-      ld2(r + p.col[k] * sv + 2 * s, a, b);
-      acc0 = mk<R>(fma(w, a.re, acc0.re), fma(w, a.im, acc0.im));
-      acc1 = mk<R>(fma(w, b.re, acc1.re), fma(w, b.im, acc1.im));
-    }
-    st2(z + t * sv + 2 * s, acc0, acc1);
-  }
-}
-
-// The same product, one block per (128-byte column of sites, right-hand side):
-// 16 complex64 or 8 complex128 sites, 8 threads of 16 bytes per row.  The
-// column's r rows are read once, coalesced, into shared memory.  Each thread
-// then forms C consecutive output rows of its 16 bytes.  Where every one of
-// those rows is the middle CSR row (t = Ltau/2) shifted along tau - taps
-// t-H .. t+H with the same values, as in the bulk of a banded P_tau - a
-// window of 2H+1 rows slides through registers with the taps as constants,
-// one shared-memory row read per output row; other rows run over their CSR
-// row.  Both orders of summation are the CSR order, so the two forms agree
-// bit for bit.
-template <typename R>
-struct Vec16;
+struct Tap;  // a real tap times a complex number
 template <>
-struct Vec16<float> {
-  using T = float4;
-  __device__ static T zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ static T fma(float c, T q, T a) {
-    return make_float4(fmaf(c, q.x, a.x), fmaf(c, q.y, a.y), fmaf(c, q.z, a.z), fmaf(c, q.w, a.w));
+struct Tap<float> {
+  static constexpr int ROWS = 16;
+  using V = float2;
+  unsigned long long c;  // the tap twice: one instruction for both parts
+  __device__ __forceinline__ explicit Tap(float t) { asm("mov.b64 %0, {%1, %1};" : "=l"(c) : "f"(t)); }
+  __device__ __forceinline__ V fma(V q, V a) const {
+    unsigned long long qa = *reinterpret_cast<unsigned long long*>(&q), aa = *reinterpret_cast<unsigned long long*>(&a);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(aa) : "l"(c), "l"(qa));
+    return *reinterpret_cast<V*>(&aa);
   }
 };
 template <>
-struct Vec16<double> {
-  using T = double2;
-  __device__ static T zero() { return make_double2(0., 0.); }
-  __device__ static T fma(double c, T q, T a) { return make_double2(::fma(c, q.x, a.x), ::fma(c, q.y, a.y)); }
+struct Tap<double> {
+  static constexpr int ROWS = 8;
+  using V = double2;
+  double c;
+  __device__ __forceinline__ explicit Tap(double t) : c(t) {}
+  __device__ __forceinline__ V fma(V q, V a) const { return make_double2(::fma(c, q.x, a.x), ::fma(c, q.y, a.y)); }
 };
 
-constexpr int PRE_H = 6;  // half-width of the banded form (13 taps, the builtin P_tau)
-constexpr int PRE_ROW_THREADS = 8;
+constexpr int PRE_H = 6;      // half-width of the banded form (13 taps, the builtin P_tau)
+constexpr int PRE_WARPS = 4;  // segments of tau per block
 
-inline size_t precon_band_smem(int Nt) { return (size_t)Nt * (16 * PRE_ROW_THREADS + 1); }
-
-template <typename R, int H, int C>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_precon_band(PreconArgs p) {
-  using VT = Vec16<R>;
-  using V = typename VT::T;
-  constexpr int PER = 16 / sizeof(Cx<R>);  // complex numbers per thread
-  constexpr int W = PRE_ROW_THREADS * PER;  // sites per column
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int Vs = p.L * p.L, Nt = p.Nt;
-  V* colv = reinterpret_cast<V*>(smem_raw);                                    // [Nt][8]
-  unsigned char* regular = smem_raw + sizeof(V) * PRE_ROW_THREADS * (size_t)Nt;  // [Nt]
-  const int c0 = blockIdx.x * W;
-  const size_t sv = 2 * (size_t)Vs;
-  const R* r = reinterpret_cast<const R*>(p.r) + (size_t)blockIdx.y * Nt * sv + 2 * (size_t)c0;
-  R* z = reinterpret_cast<R*>(p.z) + (size_t)blockIdx.y * Nt * sv + 2 * (size_t)c0;
-  const int j = threadIdx.x % PRE_ROW_THREADS, grp = threadIdx.x / PRE_ROW_THREADS;
-  const int ngrp = blockDim.x / PRE_ROW_THREADS;  // at most 32 chunks
-  const bool jon = j * PER < Vs - c0;
-  __shared__ unsigned irregular_chunks;
-  if (threadIdx.x == 0) irregular_chunks = 0;
-  // the column's rows stream into shared memory while the rows' form is found
-  if (jon)
-    for (int t = grp; t < Nt; t += ngrp)
-      cp_async16(colv + t * PRE_ROW_THREADS + j, reinterpret_cast<const V*>(r + t * sv) + j);
-  cp_async_commit();
-  // which rows are the middle row shifted (independent loads, no early exit)
-  const int tm = Nt / 2, km = p.row_ptr[tm];
-  bool band = Nt > 2 * H && p.row_ptr[tm + 1] - km == 2 * H + 1;
-  double vm[2 * H + 1];
-  if (band) {
+template <typename R>
+__global__ void __launch_bounds__(32 * PRE_WARPS, 4) k_precon(PreconArgs p) {
+  using V = typename Tap<R>::V;
+  constexpr int H = PRE_H, C = Tap<R>::ROWS, TAPS = 2 * H + 1;
+  constexpr unsigned ALL = 0xffffffffu;
+  __shared__ unsigned odd[PRE_WARPS];  // rows that are not the middle one
+  const int Vs = p.L * p.L, Nt = p.Nt, nchunk = (Vs + 31) / 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t rb = blockIdx.x / nchunk;
+  const int s = (blockIdx.x % nchunk) * 32 + lane;
+  const bool on = s < Vs;
+  const V* r = reinterpret_cast<const V*>(p.r) + rb * Nt * Vs + (on ? s : Vs - 1);
+  V* z = reinterpret_cast<V*>(p.z) + rb * Nt * Vs + s;
+  // the ends of tau, which take longer, first
+  const int b0 = (blockIdx.y == 0 ? gridDim.y - 1 : blockIdx.y - 1) * (PRE_WARPS * C), t0 = b0 + w * C;
+  // the segment's entries, asked for before the rows of r, behind which they would queue:
+  // if each of its rows has TAPS of them, entry lane + 32 n is tap i of row g
+  constexpr int NE = (C * TAPS + 31) / 32;
+  const int rows = min(max(Nt - t0, 0), C);
+  const int km = p.row_ptr[Nt / 2], k0 = p.row_ptr[min(t0, Nt)], kl = p.row_ptr[min(t0 + min(lane, C), Nt)];
+  const bool full = rows > 0 && p.row_ptr[Nt / 2 + 1] - km == TAPS && __all_sync(ALL, lane > rows || kl == k0 + TAPS * lane);
+  double vm = 0, ve[NE];
+  int cm = 0, ce[NE];
+  if (full) {
+    vm = p.val[km + min(lane, TAPS - 1)];
+    cm = p.col[km + min(lane, TAPS - 1)];
 #pragma unroll
-    for (int i = 0; i <= 2 * H; ++i) {
-      vm[i] = p.val[km + i];
-      band &= p.col[km + i] == tm - H + i;
+    for (int e = 0; e < NE; ++e) {
+      const int k = k0 + min(32 * e + lane, TAPS * rows - 1);
+      ve[e] = p.val[k];
+      ce[e] = p.col[k];
     }
   }
-  for (int t = threadIdx.x; t < Nt; t += blockDim.x) {
-    const int k0 = p.row_ptr[t];
-    bool ok = band && t >= H && t < Nt - H && p.row_ptr[t + 1] - k0 == 2 * H + 1;
-    if (ok) {
+  V q[C + 2 * H];
+  if (t0 >= H && t0 + C + H <= Nt) {
+    const V* r0 = r + (int64_t)(t0 - H) * Vs;
 #pragma unroll
-      for (int i = 0; i <= 2 * H; ++i) ok &= (p.col[k0 + i] == t - H + i) & (p.val[k0 + i] == vm[i]);
-    }
-    regular[t] = ok;
+    for (int k = 0; k < C + 2 * H; ++k) q[k] = r0[(int64_t)k * Vs];
+  } else {  // (rows outside tau are not used: a row that is the middle row shifted has none)
+#pragma unroll
+    for (int k = 0; k < C + 2 * H; ++k) q[k] = r[(int64_t)min(max(t0 - H + k, 0), Nt - 1) * Vs];
   }
-  cp_async_wait<0>();
-  __syncthreads();
-  // chunk grp (rows t0 .. t0+C-1) is regular when all its rows are
-  const int t0 = grp * C;
-  bool reg = t0 + C <= Nt;
-  for (int i = 0; reg && i < C; ++i) reg = regular[t0 + i];
-  if (!reg && j == 0) atomicOr(&irregular_chunks, 1u << grp);
-  __syncthreads();
-  if (!jon) return;
-  if (reg) {
-    R c[2 * H + 1];
+  unsigned mask = 0;
+  if (full) {
+    int i = lane % TAPS, g = lane / TAPS;
 #pragma unroll
-    for (int k = 0; k <= 2 * H; ++k) c[k] = (R)vm[k];
-    V w[2 * H + 1];
+    for (int e = 0; e < NE; ++e) {
+      const double want = __shfl_sync(ALL, vm, i);  // (all lanes)
+      if (ce[e] != t0 + g - H + i || ve[e] != want) mask |= 1u << g;
+      i += 32 % TAPS;
+      g += 32 / TAPS;
+      if (i >= TAPS) i -= TAPS, ++g;
+    }
+    mask = __reduce_or_sync(ALL, mask);
+    mask = __all_sync(ALL, lane >= TAPS || cm == Nt / 2 - H + lane) ? ~mask & ((1u << rows) - 1) : 0u;
+    // (taps reach outside tau in the first and last H rows)
+    if (t0 < H) mask &= ALL << (H - t0);
+    if (t0 + C > Nt - H) mask &= t0 < Nt - H ? (1u << (Nt - H - t0)) - 1 : 0u;
+  }
+  if (lane == 0) odd[w] = ~mask & ((1u << rows) - 1);
+  if (mask) {
+    const R vr = (R)vm;
+    R c[TAPS];
 #pragma unroll
-    for (int k = 0; k < 2 * H; ++k) w[k + 1] = colv[(t0 - H + k) * PRE_ROW_THREADS + j];
+    for (int k = 0; k < TAPS; ++k) c[k] = __shfl_sync(ALL, vr, k);
+    V* z0 = z + (int64_t)t0 * Vs;
 #pragma unroll
     for (int i = 0; i < C; ++i) {
+      if (!(mask >> i & 1)) continue;
+      V acc = {0, 0};
 #pragma unroll
-      for (int k = 0; k < 2 * H; ++k) w[k] = w[k + 1];
-      w[2 * H] = colv[(t0 + i + H) * PRE_ROW_THREADS + j];
-      V acc = VT::zero();
-#pragma unroll
-      for (int k = 0; k <= 2 * H; ++k) acc = VT::fma(c[k], w[k], acc);
-      __stcg(reinterpret_cast<V*>(z + (t0 + i) * sv) + j, acc);
+      for (int k = 0; k < TAPS; ++k) acc = Tap<R>(c[k]).fma(q[i + k], acc);
+      if (on) __stcg(z0 + (int64_t)i * Vs, acc);
     }
   }
-  // the rows of irregular chunks, spread over all row groups
-  const unsigned mask = irregular_chunks;
-  const int G = __popc(mask) * C;
-  for (int g = grp; g < G; g += ngrp) {
-    unsigned m = mask;
-    for (int q = 0; q < g / C; ++q) m &= m - 1;  // drop the chunks before the (g / C)-th
-    const int t = (__ffs(m) - 1) * C + g % C;
-    if (t >= Nt) continue;
-    V acc = VT::zero();
-    const int k1 = p.row_ptr[t + 1];
-#pragma unroll 4
-    for (int k = p.row_ptr[t]; k < k1; ++k) {
-      const int cc = p.col[k];
-      if ((unsigned)cc < (unsigned)Nt) acc = VT::fma((R)p.val[k], colv[cc * PRE_ROW_THREADS + j], acc);
+  __syncthreads();
+  int at = 0;  // odd rows before this one in the block
+  for (int g = 0; g < PRE_WARPS; ++g)
+    for (unsigned m = odd[g]; m; m &= m - 1, ++at) {
+      if (at % PRE_WARPS != w) continue;
+      const int t = b0 + g * C + __ffs(m) - 1, k1 = p.row_ptr[t + 1];
+      V acc = {0, 0};
+      for (int k = p.row_ptr[t]; k < k1; k += 32) {
+        const int cl = k + lane < k1 ? p.col[k + lane] : -1;
+        const R vl = k + lane < k1 ? (R)p.val[k + lane] : R(0);
+        for (int e = 0; e < min(32, k1 - k); e += 8) {
+          V qe[8];
+          int cc[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            cc[i] = __shfl_sync(ALL, cl, e + i);
+            qe[i] = r[(int64_t)min((unsigned)cc[i], (unsigned)Nt - 1) * Vs];
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const V next = Tap<R>(__shfl_sync(ALL, vl, e + i)).fma(qe[i], acc);
+            if ((unsigned)cc[i] < (unsigned)Nt) acc = next;  // else: outside the matrix
+          }
+        }
+      }
+      if (on) __stcg(z + (int64_t)t * Vs, acc);
     }
-    __stcg(reinterpret_cast<V*>(z + t * sv) + j, acc);
-  }
 }
 
 // ============================================================================
@@ -980,28 +979,10 @@ template int launch_bvec<double, double>(BvecArgs, int, cudaStream_t);
 
 template <typename R>
 int launch_precon(const PreconArgs& a, cudaStream_t st) {
-  const int Vs = a.L * a.L;
-  const size_t band_smem = precon_band_smem(a.Nt);
-  if (band_smem <= smem_limit()) {
-    // a tau column per block, staged in shared memory; 16, 32 or 64 rows a
-    // thread, so that a block has at most 256 threads
-    constexpr int W = PRE_ROW_THREADS * 16 / (int)sizeof(Cx<R>);
-    dim3 grid((Vs + W - 1) / W, a.bs);
-    if (a.Nt <= 512) {
-      if (prepare_smem(k_precon_band<R, PRE_H, 16>, band_smem)) return QEDF_ERR_CUDA;
-      k_precon_band<R, PRE_H, 16><<<grid, PRE_ROW_THREADS * ((a.Nt + 15) / 16), band_smem, st>>>(a);
-    } else if (a.Nt <= 1024) {
-      if (prepare_smem(k_precon_band<R, PRE_H, 32>, band_smem)) return QEDF_ERR_CUDA;
-      k_precon_band<R, PRE_H, 32><<<grid, PRE_ROW_THREADS * ((a.Nt + 31) / 32), band_smem, st>>>(a);
-    } else {
-      if (prepare_smem(k_precon_band<R, PRE_H, 64>, band_smem)) return QEDF_ERR_CUDA;
-      k_precon_band<R, PRE_H, 64><<<grid, PRE_ROW_THREADS * ((a.Nt + 63) / 64), band_smem, st>>>(a);
-    }
-  } else {
-    const int threads = 128;
-    dim3 grid((Vs / 2 + threads - 1) / threads, (a.Nt + a.TC - 1) / a.TC, a.bs);
-    k_precon<R><<<grid, threads, 0, st>>>(a);
-  }
+  const int64_t chunks = (int64_t)((a.L * a.L + 31) / 32) * a.bs;
+  const int rows = PRE_WARPS * Tap<R>::ROWS;
+  if (chunks > 0x7fffffff || (a.Nt + rows - 1) / rows > 65535) return QEDF_ERR_SIZE;
+  k_precon<R><<<dim3((unsigned)chunks, (a.Nt + rows - 1) / rows), 32 * PRE_WARPS, 0, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
 }
 template int launch_precon<float>(const PreconArgs&, cudaStream_t);
