@@ -12,10 +12,12 @@ order) and over tau, the spatial correlation of two bond products,
 evaluated with 2-D FFTs over (y, x).  Because the inverse transform is linear,
 the products of the transforms are summed over pairs and tau first and only
 one inverse FFT per observable remains; the reference instead transforms back
-per batch.  Pairs are processed in chunks sized by ``chunk_bytes``: per chunk
-one kernel writes both fields of every pair (``ops.bb_pair_fields``), cuFFT
-transforms them, and one kernel adds the products of the transforms into a
-double-precision k-space sum (``ops.bb_kspace_acc``).
+per batch.  One kernel forms both fields of a pair and slice, transforms them
+and adds their product into a double-precision k-space sum (``ops.bb_corr``).
+On sides that it is not compiled for, pairs are processed in chunks sized by
+``chunk_bytes``: per chunk one kernel writes both fields of every pair
+(``ops.bb_pair_fields``), cuFFT transforms them, and one kernel adds the
+products of the transforms to the sum (``ops.bb_kspace_acc``).
 
 Layouts as in the reference: eta, G_eta ``[Nrv, Ltau * Ly * Lx]`` (index
 tau Vs + x + Lx y); boson ``[1, 2, Lx, Ly, Ltau]``.  Inputs must be CUDA
@@ -33,10 +35,8 @@ class BondBond:
         self.Lx = self.Ly = Lx
         self.Ltau = Ltau
         self.chunk_bytes = int(chunk_bytes)
-        # fused=True: one-pass pair sums (ops.bb_corr, fields and transforms in
-        # shared memory) where the lattice fits that kernel.  Measured at
-        # L = 36, Ltau = 360, 64 vectors: 113 ms per correlator against 35 ms for
-        # the two-pass path (pair fields, cuFFT, k-space sum), so off by default
+        # the pair sums take one pass (ops.bb_corr) on every lattice that kernel
+        # is compiled for, with or without ``fused``
         self.fused = bool(fused)
 
     # ---- helpers ----------------------------------------------------------
@@ -58,7 +58,7 @@ class BondBond:
         Vs = self.Lx * self.Ly
         pairs = torch.combinations(torch.arange(nrv, device=e.device), r=2, with_replacement=False).to(torch.int32)
         S = torch.zeros(Vs, dtype=torch.complex128, device=e.device)
-        if self.fused and ops.bb_corr(kind, e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
+        if ops.bb_corr(kind, e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
             S = S.view(self.Ly, self.Lx) / (Vs * Vs)
             return (torch.fft.ifft2(S, norm="forward") / (len(pairs) * self.Ltau)).to(dt)
         chunk = min(65535, self._chunk(e.reshape(nrv, self.Ltau, self.Ly, self.Lx)), len(pairs))

@@ -191,8 +191,8 @@ def bb_pair_fields(kind: str, eta: torch.Tensor, g_eta: torch.Tensor, ephase: to
 def bb_corr(kind: str, eta: torch.Tensor, g_eta: torch.Tensor, ephase: torch.Tensor, ps: torch.Tensor,
             pt: torch.Tensor, Lx: int, S: torch.Tensor) -> bool:
     """S[k] += the pair sum of correlator ``kind`` over the pairs (ps, pt) and
-    all slices in one pass (fields and transforms in shared memory).  Returns
-    False without launching when the lattice does not fit the fused kernel
+    all slices in one pass (fields and transforms in registers).  Returns False
+    without launching on sides that the kernel is not compiled for
     (the caller then takes ``bb_pair_fields`` + FFTs + ``bb_kspace_acc``)."""
     prec, nrv, N, Vs, Ltau = _bb_inputs("bb_corr", eta, g_eta, ephase, Lx)
     _check_cuda(ps, pt, S)

@@ -155,3 +155,28 @@ def test_fused_pair_sums_match_two_pass(L, Lt, nrv, cdt, tol):
         a = getattr(BondBond(L, Lt, fused=True), name)(eta, G, bos)
         b = getattr(BondBond(L, Lt, fused=False), name)(eta, G, bos)
         assert float((a - b).abs().max() / b.abs().max()) < tol, name
+
+
+@pytest.mark.parametrize("L,Lt,nrv,cdt", [(4, 7, 3, torch.complex64), (6, 3, 2, torch.complex128), (8, 5, 4, torch.complex64),
+                                          (14, 4, 3, torch.complex128), (16, 3, 4, torch.complex64), (18, 2, 3, torch.complex128),
+                                          (22, 3, 3, torch.complex128), (26, 2, 4, torch.complex64), (30, 5, 3, torch.complex128),
+                                          (32, 2, 3, torch.complex128), (40, 1, 3, torch.complex64), (48, 2, 3, torch.complex64)])
+def test_one_pass_pair_sums(L, Lt, nrv, cdt):
+    """The one-pass kernel's sum over pairs and slices at the sides it is compiled
+    for, from items fewer than its blocks take, against transforms of fields
+    written with torch in complex128; a pair outside the vectors counts nothing."""
+    from qed_fermion_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(L)
+    eta, G = (torch.randn((nrv, Lt, L, L), dtype=cdt, device=DEV, generator=g) for _ in range(2))
+    ep = torch.exp(1j * 6.28 * torch.rand((Lt, L, L), dtype=torch.float64, device=DEV, generator=g)).to(cdt)
+    s, t = torch.combinations(torch.arange(nrv), r=2).to(torch.int32).to(DEV).T
+    ps, pt = torch.cat([s, s[:1]]).contiguous(), torch.cat([t, torch.full_like(t[:1], nrv)]).contiguous()
+    for kind in ("T1", "T21", "T2", "T4"):
+        S = torch.zeros(L * L, dtype=torch.complex128, device=DEV)
+        assert ops.bb_corr(kind, eta.view(nrv, -1), G.view(nrv, -1), ep, ps, pt, L, S)
+        a, b = _fields_torch(kind, *(x.to(torch.complex128) for x in (eta, G, ep)), s.long(), t.long())
+        prod = torch.fft.ifft2(a, norm="forward") * torch.fft.fft2(b, norm="backward")
+        want, size = prod.sum(dim=(0, 1)), prod.abs().sum(dim=(0, 1))
+        # each factor is a sum of L^2 terms in about 2 log2(L) + 8 roundings
+        eps = torch.finfo(cdt).eps
+        assert bool(((S.view(L, L) - want).abs() <= 16 * eps * np.log2(L * L) * (size + size.mean())).all()), kind
