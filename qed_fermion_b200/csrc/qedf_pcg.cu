@@ -177,7 +177,7 @@ size_t pcg_carve(PcgParams& p, int sloppy_bytes, void* workspace, size_t* zero_b
   p.xlo = mode_mixed(p.mode) ? take(full) : nullptr;
   p.y0 = mode_narrow(p.mode) ? take(full) : mode_mixed(p.mode) ? p.z : nullptr;
   p.acc = static_cast<double*>(take(accb));
-  p.bar = static_cast<unsigned int*>(take(barb));
+  p.bar = static_cast<unsigned long long*>(take(barb));
   p.ptab = static_cast<float*>(take(tabb));
   return at;
 }

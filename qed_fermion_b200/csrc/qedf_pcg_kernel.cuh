@@ -55,34 +55,33 @@ namespace qedf {
 // ---------------------------------------------------------------------------
 // bounded grid barrier
 // ---------------------------------------------------------------------------
-// bar[0] counts arrivals over the whole solve (zeroed per solve); barrier n
-// of a block is passed once the count reaches n * nblocks.  Arrival is a
-// release reduction without a reply, and waiting an acquire load of the
+// The low half of *bar counts arrivals over the whole solve (zeroed per solve);
+// barrier n of a block is passed once the count reaches n * nblocks.  Arrival is
+// a release reduction without a reply, and waiting an acquire load of the
 // count, so the last block's arrival ends the barrier directly (release and
 // acquire at GPU scope, ordered after and before the block barriers, need no
-// further fences).  bar[2] is
-// the error word.  `target` is the calling block's count to wait for, kept
+// further fences).  The high half is the error word: read apart, it doubled the
+// time between two looks at the count and followed the last of them.  `target` is the calling block's count to wait for, kept
 // by its thread 0 across calls.
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int nblocks, long long budget,
+__device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned int nblocks, long long budget,
                                              unsigned int& target) {
   __syncthreads();
   int ok = 1;
   if (threadIdx.x == 0) {
-    volatile unsigned int* err = bar + 2;
     target += nblocks;
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;\n" ::"l"(bar), "r"(1u) : "memory");
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;\n" ::"l"(bar), "l"(1ull) : "memory");
     const long long t0 = clock64();
     while (true) {
-      unsigned int v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(bar) : "memory");
-      if ((int)(v - target) >= 0) break;
-      if (*err) break;
+      unsigned long long w;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(w) : "l"(bar) : "memory");
+      ok = (w >> 32) == 0;
+      if (!ok || (int)((unsigned int)w - target) >= 0) break;
       if (clock64() - t0 > budget) {
-        atomicExch(bar + 2, (unsigned int)QEDF_ERR_TIMEOUT);
+        atomicOr(bar, (unsigned long long)QEDF_ERR_TIMEOUT << 32);
+        ok = 0;
         break;
       }
     }
-    ok = *err == 0;
   }
   return __syncthreads_and(ok);
 }
@@ -93,27 +92,31 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// three sums over the block at once, results valid in thread 0 (sh: 96 doubles)
-__device__ __forceinline__ void block_sum3_d(double& a, double& b, double& c, double* sh) {
+// sums over the block, results valid in thread 0 (sh: 32 doubles each)
+__device__ __forceinline__ void block_sum_d(double& a, double* sh) {
+  a = warp_sum_d(a);
+  const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  __syncthreads();
+  if (ln == 0) sh[w] = a;
+  __syncthreads();
+  if (threadIdx.x < 32) a = warp_sum_d(threadIdx.x < (blockDim.x + 31) / 32 ? sh[threadIdx.x] : 0.0);
+}
+__device__ __forceinline__ void block_sum2_d(double& a, double& b, double* sh) {
   a = warp_sum_d(a);
   b = warp_sum_d(b);
-  c = warp_sum_d(c);
   const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
   __syncthreads();
   if (ln == 0) {
     sh[w] = a;
     sh[32 + w] = b;
-    sh[64 + w] = c;
   }
   __syncthreads();
   if (threadIdx.x < 32) {
     const bool in = threadIdx.x < (blockDim.x + 31) / 32;
     a = warp_sum_d(in ? sh[threadIdx.x] : 0.0);
     b = warp_sum_d(in ? sh[32 + threadIdx.x] : 0.0);
-    c = warp_sum_d(in ? sh[64 + threadIdx.x] : 0.0);
   }
 }
-
 // ---------------------------------------------------------------------------
 // accumulator layout (doubles)
 // ---------------------------------------------------------------------------
@@ -544,7 +547,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
   constexpr bool H16 = std::is_same<SP, __half>::value;
   constexpr bool LOWP = !std::is_same<SP, RS>::value;
   extern __shared__ __align__(128) unsigned char dsm_all[];
-  __shared__ double red[96];
+  __shared__ double red[64];
   __shared__ PcgCtl ctl;
   __shared__ OpRun<RS, A, SP> oprun;
 #define NV p.nrhs
@@ -677,7 +680,8 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     RS* rout = rbuf(kind == 1 ? ctl.rcur ^ 1 : ctl.rcur);
     const RS* Op = reinterpret_cast<const RS*>(p.Op);
     SP* z = reinterpret_cast<SP*>(p.z);
-    const RS al = (RS)st.alpha()[v];
+    // (alpha from its accumulator, whose latency is then the rows' own)
+    const RS al = kind != 1 ? (RS)0 : ctl.guess ? (RS)1 : (RS)(st.rz()[v] / acc.pAp(ctl.it & 1)[v]);
     RS cpart = 0;
     // row i of the column is slice t0 - h + i (mod Nt); the unit's own rows are [h, h + len)
     auto slice_of = [&](int i) {
@@ -821,7 +825,8 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     double a = 0, b = 0, c = 0;
     for_units([&](int v, const PcgSys& S, int u) { elementwise(kind_c, v, S, u, a, b, c); },
               [&](int v) {
-                block_sum3_d(a, b, c, red);
+                if (kind == 0) block_sum_d(a, red);
+                block_sum2_d(b, c, red);
                 if (tid == 0) {
                   if (kind == 0) atomicAdd(acc.bb() + v, a);
                   if (kind == 0 || kind == 1) atomicAdd(acc.rr(slot) + v, c);
@@ -835,7 +840,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
   // ---- operator pass over this block's runs of slices ------------------------------
     auto operator_pass = [&](int slot) {
     for_slices([&](int v, const PcgSys& S, int a, int b) {
-      double pap = 0, ppp = 0, none = 0;
+      double pap = 0, ppp = 0;
       __syncthreads();
       if (tid == 0) {
         const int64_t vb = 2 * vec_base(S, v);  // reals
@@ -871,7 +876,8 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
       }
       __syncthreads();
       if (tid < p.eng_threads) operator_run<RS, A, SP, BY>(oprun, dsm, pap, ppp);
-      block_sum3_d(pap, ppp, none, red);
+      if constexpr (H16) block_sum2_d(pap, ppp, red);
+      else block_sum_d(pap, red);
       if (tid == 0) {
         atomicAdd(acc.pAp(slot) + v, pap);
         if constexpr (H16) atomicAdd(acc.pp(slot) + v, ppp);
@@ -957,6 +963,8 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
       if (acc.bb()[v] == 0.0) {  // b = 0: x = 0 is exact
         st.active()[v] = 0;
         st.res()[v] = 0.0;
+      } else {
+        st.res()[v] = sqrt(st.rr()[v] / acc.bb()[v]);
       }
     }
     __syncthreads();
@@ -997,8 +1005,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     for (int v = tid; v < NV; v += blockDim.x) {
       st.ru()[v] = 0;
       if (!st.active()[v]) continue;
-      const double res = sqrt(st.rr()[v] / acc.bb()[v]);
-      st.res()[v] = res;
+      const double res = st.res()[v];
       if (!isfinite(res)) {
         st.active()[v] = 0;
         st.status()[v] = QEDF_ERR_NAN;
@@ -1038,12 +1045,12 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
         });
         if (!(ok = barrier())) break;
         for_slices([&](int v, const PcgSys& S, int a, int b) {
-          double sum = 0, n1 = 0, n2 = 0;
+          double sum = 0;
           if (tid < p.eng_threads) {
             const TrueRun<RS, RH, A> q = true_run(v, S, a, b);
             sum = true_residual_run<RS, RH, A, BY, true>(q, (int)RhsState::bytes(NV));
           }
-          block_sum3_d(sum, n1, n2, red);
+          block_sum_d(sum, red);
           if (tid == 0) atomicAdd(acc.ru_rr() + v, sum);
         });
         if (!(ok = barrier())) break;
@@ -1123,7 +1130,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
         st.alpha()[v] = ctl.guess ? 1.0 : st.rz()[v] / acc.pAp(aslot)[v];
         if constexpr (H16) st.scz()[v] = st_scale(st.rr()[v]);  // |r| before this update
       }
-    __syncthreads();
+    if constexpr (H16) __syncthreads();
     elementwise_pass(std::integral_constant<int, 1>(), ctl.slot ^ 1);
     if (blockIdx.x == 0)  // pAp (and |p|^2) slot of the next iteration
       for (int v = tid; v < NV; v += blockDim.x) {
@@ -1139,6 +1146,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
       st.rzold()[v] = st.rz()[v];
       st.rz()[v] = acc.rz(slot)[v];
       st.rr()[v] = acc.rr(slot)[v];
+      st.res()[v] = sqrt(st.rr()[v] / acc.bb()[v]);
       if (ctl.guess) continue;
       st.iters()[v] += 1;
       st.pending()[v] = 1;
@@ -1161,7 +1169,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     fold_pass();
   }
   if (blockIdx.x == 0) {
-    const unsigned int err = *((volatile unsigned int*)(p.bar + 2));
+    const unsigned int err = (unsigned int)(*((volatile unsigned long long*)p.bar) >> 32);
     for (int v = tid; v < NV; v += blockDim.x) {
       int stt = st.status()[v];
       if (err) stt = (int)err;
