@@ -216,14 +216,10 @@ struct PcgT {
   static constexpr bool TALL = sizeof(RS) == 8 && BY >= 4;
   static constexpr bool IN_OP = sizeof(RS) == 8;  // y_t waits in Op
   // x_lo or the angles of the next slice are on their way into shared memory
-  // while B is applied (loaded when needed, their latency is exposed), and with
-  // tall tiles z and p_old too: these fit in registers beside the tile only at
-  // BY = 2 (operator phase at L = 48, 2 right-hand sides: 62 K cycles, 70 K
-  // through shared memory), and spills are dear, since shared memory leaves
-  // little L1 for them (BY = 6: 75 K cycles through shared memory, 81 K spilled).
+  // while B is applied (loaded when needed, their latency is exposed); z and
+  // p_old go to registers (operator phase at L = 48, 2 right-hand sides: 62 K
+  // cycles, 70 K through shared memory).
   static constexpr bool STAGE = !TALL;
-  static constexpr bool STAGE_ZP = false;
-  static constexpr bool EARLY = false;
   static constexpr bool PHS = IN_OP;
   static constexpr int threads = MaxT<RS, BY>::value;
   // 80 registers at BY = 2: two 384-thread blocks per SM
@@ -273,8 +269,7 @@ template <typename RS, typename RH, typename SP, int BY>
 inline size_t pcg_phase_smem(int eng_threads, int col_rows, int CH) {
   using T = PcgT<RS, BY>;
   size_t s = slice_smem<RS>(eng_threads, Slice<RS, BY, T::PHS, T::TALL ? 1 : 2>::REC) +
-             (T::IN_OP ? 0 : 2 * stash_smem<RS, BY>(eng_threads)) + (T::STAGE ? (T::EARLY ? 2 : 1) * TileSlot<RS, BY>::smem(eng_threads) : 0) +
-             (T::STAGE_ZP ? 2 * TileSlot<SP, BY>::smem(eng_threads) : 0);
+             (T::IN_OP ? 0 : 2 * stash_smem<RS, BY>(eng_threads)) + (T::STAGE ? TileSlot<RS, BY>::smem(eng_threads) : 0);
   if (!std::is_same<RS, RH>::value) s = std::max(s, slice_smem<RH>(eng_threads, Slice<RH, BY, true, 1>::REC));
   return std::max(s, sizeof(Cx<RS>) * (size_t)col_rows * CH);
 }
@@ -304,52 +299,43 @@ __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned
   using CT = PcgT<RS, BY>;
   constexpr bool H16 = std::is_same<SP, __half>::value, LOWP = !std::is_same<SP, RS>::value;
   using Eng = Slice<RS, BY, CT::PHS, CT::TALL ? 1 : 2>;
+  // the first two slices' angles are asked for together: at BY = 2, where
+  // registers hold them, 2 to 4 % of an iteration (L = 48, 2 right-hand sides,
+  // 53.6 -> 52.3 us); with taller tiles or converted storage they spill
+  constexpr bool AHEAD = sizeof(RS) == 4 && BY == 2 && !LOWP;
   const int tid = threadIdx.x;
   Eng E;
   E.init_named(q.L, smem, tid, q.eng);
   size_t at = slice_smem<RS>(q.eng, Eng::REC);
-  // y_t and y_{t+1} wait in two stashes in turn; with STAGE_ZP the one that is
-  // free at the time holds z
+  // y_t and y_{t+1} wait in two stashes in turn
   Stash<RS, BY> stash, other;
   if constexpr (!CT::IN_OP) {
-    static_assert(TileSlot<RS, BY>::BYTES == stash_record<RS, BY>() * sizeof(Cx<RS>), "a stash holds z");
     stash.init(smem + at, tid);
     at += stash_smem<RS, BY>(q.eng);
     other.init(smem + at, tid);
     at += stash_smem<RS, BY>(q.eng);
   }
-  TileSlot<A, BY> slot_a, slot_x;  // the angles; x (one slot for both in turn unless EARLY)
+  TileSlot<A, BY> slot;  // the angles and x in turn
   static_assert(sizeof(A) == sizeof(RS), "x and the angles share a slot");
-  if constexpr (CT::STAGE) slot_a.init(smem + at, tid);
-  if constexpr (CT::STAGE) slot_x.init(smem + at + (CT::EARLY ? TileSlot<RS, BY>::smem(q.eng) : 0), tid);
-  TileSlot<SP, BY> slot_z, slot_p;
-  if constexpr (CT::STAGE_ZP) {
-    at += TileSlot<RS, BY>::smem(q.eng);
-    slot_z.init(smem + at, tid);
-    slot_p.init(smem + at + TileSlot<SP, BY>::smem(q.eng), tid);
-  }
+  if constexpr (CT::STAGE) slot.init(smem + at, tid);
   const int a = q.a;
   double pap = 0, ppp = 0;
   Cx<RS> X0[BY][2], X1[BY][2], Y[BY][2];
   // z and p_old of slice t, and x of own slices with a pending update, on their way
   auto fetch = [&](Cx<RS> (&X)[BY][2], Cx<RS> (&T)[BY][2], int t, bool own) {
     if constexpr (CT::STAGE) {
-      if constexpr (CT::STAGE_ZP) {
-        slot_z.fetch(q.zz + t * q.sv + E.off, E.rs);
-        slot_p.fetch(q.pold + t * q.sv + E.off, E.rs);
-      }
-      if (own && q.x_too) slot_x.fetch_first(q.xl + t * q.sv + E.off, E.rs);
+      if (own && q.x_too) slot.fetch_first(q.xl + t * q.sv + E.off, E.rs);
       cp_async_commit();
     }
-    if constexpr (!CT::STAGE_ZP) {
-      E.load_st(X, q.zz + t * q.sv, q.s_z);
-      E.load_st(T, q.pold + t * q.sv, q.s_po);
-    }
+    E.load_st(X, q.zz + t * q.sv, q.s_z);
+    E.load_st(T, q.pold + t * q.sv, q.s_po);
   };
   // the angles of slice t on their way, where x waited
   auto fetch_angles = [&](int t) {
-    slot_a.fetch_first(q.phi + t * q.sv + E.off, E.rs);
-    cp_async_commit();
+    if constexpr (CT::STAGE) {
+      slot.fetch_first(q.phi + t * q.sv + E.off, E.rs);
+      cp_async_commit();
+    }
   };
   auto phases = [&](int t) {
     A ang[BY][4];
@@ -358,7 +344,7 @@ __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned
 #pragma unroll
       for (int r = 0; r < BY; ++r) {
         Cx<A> u, w;
-        ld2c(slot_a.row(r), u, w);
+        ld2c(slot.row(r), u, w);
         ang[r][0] = u.re;
         ang[r][1] = u.im;
         ang[r][2] = w.re;
@@ -376,16 +362,7 @@ __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned
 #pragma unroll
     for (int r = 0; r < BY; ++r) {
       const int64_t i = t * q.sv + E.off + r * E.rs;
-      Cx<RS> Z0, Z1, T0, T1;
-      if constexpr (CT::STAGE_ZP) {
-        ld2s(slot_z.row(r), Z0, Z1, q.s_z);
-        ld2s(slot_p.row(r), T0, T1, q.s_po);
-      } else {
-        Z0 = Z[r][0];
-        Z1 = Z[r][1];
-        T0 = T[r][0];
-        T1 = T[r][1];
-      }
+      const Cx<RS> Z0 = Z[r][0], Z1 = Z[r][1], T0 = T[r][0], T1 = T[r][1];
       X[r][0] = mk<RS>(fma(q.beta, T0.re, Z0.re), fma(q.beta, T0.im, Z0.im));
       X[r][1] = mk<RS>(fma(q.beta, T1.re, Z1.re), fma(q.beta, T1.im, Z1.im));
       if constexpr (LOWP) {
@@ -396,7 +373,7 @@ __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned
       if (E.on) st2s(q.pnew + i, X[r][0], X[r][1], q.i_pn);
       if (q.x_too) {
         Cx<RS> l0, l1;
-        if constexpr (CT::STAGE) ld2c(slot_x.row(r), l0, l1);
+        if constexpr (CT::STAGE) ld2c(slot.row(r), l0, l1);
         else ld2c(q.xl + i, l0, l1);
         l0 = mk<RS>(fma(q.al_old, T0.re, l0.re), fma(q.al_old, T0.im, l0.im));
         l1 = mk<RS>(fma(q.al_old, T1.re, l1.re), fma(q.al_old, T1.im, l1.im));
@@ -407,34 +384,30 @@ __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned
       if (own && E.on) ppp += sq_blk<RS, BY>(X);
   };
   const int tp = a == 0 ? q.Nt - 1 : a - 1;
-  // z and p_old of the slice after this one; with EARLY they are under way for
-  // two B's, else for one
-  Cx<RS> Z[BY][2], T[BY][2];
-  auto next = [](int t, int Nt) { return t >= Nt ? t - Nt : t; };
-  if constexpr (CT::STAGE) fetch_angles(tp);
+  Cx<RS> Z[BY][2], T[BY][2];  // z and p_old of the slice after this one
+  A first[BY][4];             // the angles of the first slice
+  fetch_angles(tp);
   fetch(Z, T, tp, false);
+  if constexpr (AHEAD) E.load_angles(first, q.phi + a * q.sv);
   phases(tp);
   form(X0, Z, T, tp, false);
   fetch(Z, T, a, true);
   E.template applyB<0>(X0);
+  if constexpr (AHEAD) E.phases(first, q.t1, q.th);
   form(X1, Z, T, a, true);
-  if constexpr (CT::STAGE) fetch_angles(a);
-  if constexpr (CT::EARLY) fetch(Z, T, next(a + 1, q.Nt), a + 1 < q.b);
+  if constexpr (!AHEAD) fetch_angles(a);
   axpy_blk<RS, BY>(Y, X1, sigma_of<RS>(tp, q.Nt) * q.Cb, X0);  // y_a
   if constexpr (CT::IN_OP) E.store(q.O + a * q.sv, Y); else stash.park(Y);
   copy_blk<RS, BY>(X0, X1);
   for (int t = a; t < q.b; ++t) {
     const int tn = t + 1 == q.Nt ? 0 : t + 1;
     const bool own = t + 1 < q.b;
-    phases(t);
+    if (!AHEAD || t > a) phases(t);
     const RS sg = sigma_of<RS>(t, q.Nt) * q.Cb;
-    if constexpr (!CT::EARLY) fetch(Z, T, tn, own);
+    fetch(Z, T, tn, own);
     E.template applyB<1>(X0);            // B_t p_t
     form(X1, Z, T, tn, own);
-    if constexpr (CT::STAGE)
-      if (own) fetch_angles(t + 1);
-    if constexpr (CT::EARLY)
-      if (own) fetch(Z, T, next(t + 2, q.Nt), t + 2 < q.b);
+    if (own) fetch_angles(t + 1);
     axpy_blk<RS, BY>(Y, X1, sg, X0);     // y_{t+1}
     // y_t and y_{t+1} are not in registers now
     if constexpr (CT::IN_OP) {
