@@ -23,6 +23,11 @@ static bool mode_mixed(int mode) {
 }
 static bool mode_narrow(int mode) { return mode == QEDF_PCG_MIXED_BF16 || mode == QEDF_PCG_MIXED_F16; }
 
+// slices of side L that an SM holds, by the warps that the kernels' registers allow
+static int resident_slices(int L, int by) {
+  return std::min(PCG_MAX_PER_SM, (by == 2 ? 20 : 16) / std::max(4, slice_threads(L, by) / 32));
+}
+
 // Tau segments of the elementwise units: whole tau columns (one segment) where
 // these fill the GPU, else as many segments as shorten the busiest block's
 // work, counted in rows with twelve rows of the neighbours and about forty
@@ -58,14 +63,22 @@ int pcg_plan(PcgParams& p, const qedf_system* sys, int nsys, const qedf_pcg_opts
   const bool wide_fits = o->mode != QEDF_PCG_PLAIN_F64 && ntmax_all <= 500;
   if (o->chunk == 32 && !wide_fits) return QEDF_ERR_SIZE;
   p.CH = o->chunk ? o->chunk : PCG_CHUNK;
-  int64_t columns = 0, elements = 0;
+  int Lmax = 0;
+  int64_t columns = 0, elements = 0, slices = 0;
   for (int s = 0; s < nsys; ++s) {
     const qedf_system& q = sys[s];
     if (q.Lx < 2 || q.Lx % 2 || q.Ltau < 2 || q.nrhs < 1) return QEDF_ERR_ARG;
     columns += (int64_t)q.nrhs * (((int64_t)q.Lx * q.Lx + p.CH - 1) / p.CH);
     elements += (int64_t)q.nrhs * q.Ltau * q.Lx * q.Lx;
+    Lmax = std::max(Lmax, q.Lx);
+    slices += (int64_t)q.nrhs * q.Ltau;
   }
   const bool may_split = elements * 2 * pcg_storage_bytes(o->mode) <= 9000000;
+  // blocks that take them: two per SM, or as many as the operator's slices bring
+  // and fit (double precision, whose units take twice as long: L = 20, 3
+  // right-hand sides, 36.9 -> 33.2 us per iteration; L = 24, 2: 35.2 -> 33.2)
+  const int64_t seg_most = (int64_t)num_sms() * std::max(2, resident_slices(Lmax, 2));
+  const int seg_blocks = (int)std::min(std::max<int64_t>(slices, 2 * num_sms()), seg_most);
   int rhs = 0, pt = 0;
   int64_t vec = 0, phi = 0;
   for (int s = 0; s < nsys; ++s) {
@@ -101,7 +114,7 @@ int pcg_plan(PcgParams& p, const qedf_system* sys, int nsys, const qedf_pcg_opts
     }
     S.nslab = (q.Ltau + S.T - 1) / S.T;
     S.nchunk = (q.Lx * q.Lx + p.CH - 1) / p.CH;
-    S.nseg = may_split ? auto_segments(columns, q.Ltau, 2 * num_sms()) : 1;
+    S.nseg = may_split ? auto_segments(columns, q.Ltau, seg_blocks) : 1;
     S.seg = (q.Ltau + S.nseg - 1) / S.nseg;
     S.nseg = (q.Ltau + S.seg - 1) / S.seg;
     if (S.nseg > 1) p.split = 1;
@@ -328,8 +341,7 @@ static int pcg_pick_by(const PcgParams& p) {
     bool ok = true;
     for (int s = 0; s < p.nsys; ++s) ok = ok && by_valid(p.sys[s].L, by);
     if (!ok || (by == 6 && best > 0)) continue;
-    const int warps = std::max(4, slice_threads(Lmax, by) / 32);
-    const int n = std::min(PCG_MAX_PER_SM, (by == 2 ? 20 : 16) / warps);
+    const int n = resident_slices(Lmax, by);
     if (best < 0 || n > most) {
       best = by;
       most = n;
