@@ -12,13 +12,17 @@
 //
 // The double-precision pipe and the shared memory's 16-byte exchanges bound it.
 // Measured against pair fields in memory, cuFFT and a k-space sum, 20 vectors
-// and Ltau = 10 L, whole calls with 0.2 ms of host work: L = 30, complex128,
+// and Ltau = 10 L, one correlator with 0.2 ms of host work: L = 30, complex128,
 // 2.2 -> 1.1 ms, complex64 1.5 -> 0.6 ms; L = 20, 0.86 -> 0.39 and 0.58 -> 0.33;
 // L = 48, complex64, 12 vectors, 2.0 -> 1.5 ms.  Lines of more than 32 sites in
-// double precision leave one line per thread no registers (L = 36: 1.33 against
-// 1.31 ms), so they keep the two passes.  Blocks per SM: at L = 30, complex128,
-// two with 255 registers a thread take 1.1 ms, three with 168 1.35 ms: the
-// shared memory of the third is L1 that the vectors' slices need.
+// double precision leave one line per thread few registers (one correlator at
+// L = 36: 1.33 against 1.31 ms), so a single correlator keeps the two passes
+// there.  Blocks per SM: at L = 30, complex128, two with 255 registers a thread
+// take 1.1 ms, three with 168 1.35 ms: the shared memory of the third is L1 that
+// the vectors' slices need.  The sum of all four, in place of T1, T21 and T4 in
+// turn: L = 30, 20 vectors, complex128 3.6 -> 1.65 ms, complex64 2.2 -> 0.95; L =
+// 20, 1.5 -> 0.64 and 1.15 -> 0.51; L = 48, complex64, 12 vectors, 5.2 -> 1.5; L =
+// 36, complex128, 12 vectors, 4.4 -> 1.5; L = 40, 6.8 -> 2.0.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -182,20 +186,32 @@ struct Line {
   }
 };
 
-constexpr int CORR_THREADS = 128;
+// fields of a pair and slice: two of one correlator, or the four of all
+constexpr int CORR_ONE = 2, CORR_ALL = 4;
+constexpr int corr_threads(int L, int NF) { return NF * L <= 128 ? 128 : (NF * L + 31) / 32 * 32; }
 constexpr int CORR_CLUSTER = 8;  // blocks that add up their sums (the portable size)
-// blocks per SM that leave a thread the registers of its line
-constexpr int corr_blocks(int L, int words) { return L * words <= 40 ? 4 : L * words <= 48 ? 3 : 2; }
+// blocks per SM that leave a thread the registers of its line and fit in shared memory
+constexpr int corr_blocks(int L, int words, int NF) {
+  if (NF == CORR_ALL && words == 1) return L <= 32 ? 4 : L <= 36 ? 3 : 2;
+  if (L * words > 72) return 1;
+  return L * words <= 40 ? 4 : L * words <= 48 ? 3 : 2;
+}
 
-template <typename R, int P, int Q>
-__global__ void __launch_bounds__(CORR_THREADS, corr_blocks(P * Q, sizeof(R) / 4)) k_bb_corr(BondArgs a, int ni,
-                                                                                        double* S) {
+// NF = CORR_ALL: the sum of all four correlators, whose fields are sums of the
+// same four: U_st(r) = conj(eta_s(r)) G_t(r + x) e^{i phi}, V_st(r) = conj(eta_s(r
+// + x)) G_t(r) e^{-i phi}, and U_ts, V_ts.  T1 correlates U_st with U_ts, T4 V_st
+// with V_ts, T21 (V_st + V_ts) / 2 with (U_st + U_ts) / 2, and T2 is T21 at -k.
+// So four transforms do instead of six in three launches, one sum instead of
+// three, and A(k), the transform of U_st at -k, needs no conjugation.
+template <typename R, int P, int Q, int NF>
+__global__ void __launch_bounds__(corr_threads(P* Q, NF), corr_blocks(P* Q, sizeof(R) / 4, NF))
+    k_bb_corr(BondArgs a, int ni, double* S) {
   constexpr int L = P * Q, Vs = L * L, PITCH = L | 1;  // rows apart by an odd number of complex numbers
   using T = Line<R, P, Q>;
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* sum = reinterpret_cast<double2*>(smraw);   // [Vs]
-  Cx<R>* F = reinterpret_cast<Cx<R>*>(sum + Vs);      // [ni][2][L][PITCH]
-  Cx<R>* tw = F + (size_t)ni * 2 * L * PITCH;         // [L]
+  Cx<R>* F = reinterpret_cast<Cx<R>*>(sum + Vs);      // [ni][NF][L][PITCH]
+  Cx<R>* tw = F + (size_t)ni * NF * L * PITCH;        // [L]
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int i = tid; i < L; i += nt) {
     double sn, cs;
@@ -204,13 +220,13 @@ __global__ void __launch_bounds__(CORR_THREADS, corr_blocks(P * Q, sizeof(R) / 4
   }
   for (int i = tid; i < Vs; i += nt) sum[i] = make_double2(0, 0);
   __syncthreads();
-  // this thread's item of the block's ni, its field (a or b) and line
-  const int it = tid / (2 * L), f = tid / L & 1, l = tid % L;
+  // this thread's item of the block's ni, its field (a or b, st or ts) and line
+  const int it = tid / (NF * L), f = tid / L & 1, l = tid % L;
   const bool mine = it < ni;
   Cx<R>* Ff = F + (size_t)(tid / L) * L * PITCH;
-  const bool two = a.kind == 21 || a.kind == 2;
+  const bool two = NF == CORR_ONE && (a.kind == 21 || a.kind == 2);
   // conj(eta) at r, G at r + x, times e^{i phi}; else conj(eta) at r + x, G at r, times e^{-i phi}
-  const bool up = a.kind == 1 || (a.kind == 21 && f) || (a.kind == 2 && !f);
+  const bool up = NF == CORR_ALL ? (tid / L & 2) == 0 : a.kind == 1 || (a.kind == 21 && f) || (a.kind == 2 && !f);
   const int l1 = l + 1 == L ? 0 : l + 1;
   const R* eta = reinterpret_cast<const R*>(a.eta) + 2 * (up ? l : l1);
   const R* g = reinterpret_cast<const R*>(a.g) + 2 * (up ? l1 : l);
@@ -238,7 +254,7 @@ __global__ void __launch_bounds__(CORR_THREADS, corr_blocks(P * Q, sizeof(R) / 4
           Cx<R> e = ldcx(ep, sl + y * L);
           if (!up) e = conjc(e);
           v = cmul(v, e);
-          x[y] = f ? v : conjc(v);
+          x[y] = f || NF == CORR_ALL ? v : conjc(v);
         }
       }
       T::run(x, tw, [&](int k, Cx<R> v) { Ff[k * PITCH + l] = v; });
@@ -252,16 +268,51 @@ __global__ void __launch_bounds__(CORR_THREADS, corr_blocks(P * Q, sizeof(R) / 4
       T::run(x, tw, [&](int k, Cx<R> v) { row[k] = v; });
     }
     __syncthreads();
-    for (int k = tid; k < Vs; k += nt) {
-      const Cx<R>* q = F + k / L * PITCH + k % L;
-      double2 c = sum[k];
-      for (int i = 0; i < n; ++i, q += 2 * L * PITCH) {
-        const Cx<R> u = q[0], v = q[L * PITCH];
-        const double ur = u.re, ui = -u.im, vr = v.re, vi = v.im;
-        c.x = fma(ur, vr, fma(-ui, vi, c.x));
-        c.y = fma(ur, vi, fma(ui, vr, c.y));
+    if constexpr (NF == CORR_ALL) {
+      // k and -k together: rows up to L / 2, of the first and the last row half
+      for (int k = tid; k < (L / 2 + 1) * L; k += nt) {
+        const int ky = k / L, kx = k % L;
+        if (ky % (L / 2) == 0 && kx > L / 2) continue;
+        const int my = ky ? L - ky : 0, mx = kx ? L - kx : 0, m = my * L + mx;
+        const Cx<R>*q = F + ky * PITCH + kx, *r = F + my * PITCH + mx;
+        double2 c = sum[k], d = sum[m];
+        auto at = [](const Cx<R>* u, int j) {
+          const Cx<R> v = u[j * L * PITCH];
+          return make_double2(v.re, v.im);
+        };
+        auto add = [](double2& s, double2 u, double2 v) {
+          s.x = fma(u.x, v.x, fma(-u.y, v.y, s.x));
+          s.y = fma(u.x, v.y, fma(u.y, v.x, s.y));
+        };
+        for (int i = 0; i < n; ++i, q += NF * L * PITCH, r += NF * L * PITCH) {
+          double2 u = at(q, 0), w = at(q, 1), um = at(r, 0), wm = at(r, 1);  // U_st, U_ts at k and -k
+          add(c, um, w);
+          add(d, u, wm);
+          const double2 U = make_double2(u.x + w.x, u.y + w.y), Um = make_double2(um.x + wm.x, um.y + wm.y);
+          u = at(q, 2), w = at(q, 3), um = at(r, 2), wm = at(r, 3);  // V_st, V_ts
+          add(c, um, w);
+          add(d, u, wm);
+          double2 e = make_double2(0, 0);
+          add(e, make_double2(um.x + wm.x, um.y + wm.y), U);
+          add(e, make_double2(u.x + w.x, u.y + w.y), Um);
+          c = make_double2(fma(0.25, e.x, c.x), fma(0.25, e.y, c.y));
+          d = make_double2(fma(0.25, e.x, d.x), fma(0.25, e.y, d.y));
+        }
+        sum[k] = c;
+        if (m != k) sum[m] = d;
       }
-      sum[k] = c;
+    } else {
+      for (int k = tid; k < Vs; k += nt) {
+        const Cx<R>* q = F + k / L * PITCH + k % L;
+        double2 c = sum[k];
+        for (int i = 0; i < n; ++i, q += 2 * L * PITCH) {
+          const Cx<R> u = q[0], v = q[L * PITCH];
+          const double ur = u.re, ui = -u.im, vr = v.re, vi = v.im;
+          c.x = fma(ur, vr, fma(-ui, vi, c.x));
+          c.y = fma(ur, vi, fma(ui, vr, c.y));
+        }
+        sum[k] = c;
+      }
     }
     __syncthreads();
   }
@@ -283,12 +334,12 @@ __global__ void __launch_bounds__(CORR_THREADS, corr_blocks(P * Q, sizeof(R) / 4
   cluster.sync();  // no block's shared memory goes while another reads it
 }
 
-template <typename R, int P, int Q>
+template <typename R, int NF, int P, int Q>
 static int launch_corr_pq(const BondArgs& a, double* S, cudaStream_t st) {
   constexpr int L = P * Q;
-  const int ni = std::max(1, CORR_THREADS / (2 * L)), threads = (ni * 2 * L + 31) / 32 * 32;
-  const size_t smem = L * L * sizeof(double2) + ((size_t)ni * 2 * L * (L | 1) + L) * sizeof(Cx<R>);
-  if (cudaFuncSetAttribute(k_bb_corr<R, P, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  const int ni = corr_threads(L, NF) / (NF * L), threads = (ni * NF * L + 31) / 32 * 32;
+  const size_t smem = L * L * sizeof(double2) + ((size_t)ni * NF * L * (L | 1) + L) * sizeof(Cx<R>);
+  if (cudaFuncSetAttribute(k_bb_corr<R, P, Q, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return QEDF_ERR_CUDA;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -302,49 +353,56 @@ static int launch_corr_pq(const BondArgs& a, double* S, cudaStream_t st) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int clusters = 0;  // that are resident at a time
-  if (cudaOccupancyMaxActiveClusters(&clusters, k_bb_corr<R, P, Q>, &cfg) != cudaSuccess || clusters < 1)
+  if (cudaOccupancyMaxActiveClusters(&clusters, k_bb_corr<R, P, Q, NF>, &cfg) != cudaSuccess || clusters < 1)
     return QEDF_ERR_SIZE;
   const int64_t per = (int64_t)ni * CORR_CLUSTER, want = ((int64_t)a.npairs * a.Nt + per - 1) / per;
   cfg.gridDim = CORR_CLUSTER * (unsigned)std::min<int64_t>(want, clusters);
-  if (cudaLaunchKernelEx(&cfg, k_bb_corr<R, P, Q>, a, ni, S) != cudaSuccess) return QEDF_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, k_bb_corr<R, P, Q, NF>, a, ni, S) != cudaSuccess) return QEDF_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
 }
 
-// even sides whose factors have transforms and whose lines fit in registers
-template <typename R>
+// even sides (the sum of all takes k and -k together) whose factors have transforms and whose lines fit in registers
+template <typename R, int NF>
 static int launch_corr(const BondArgs& a, double* S, cudaStream_t st) {
   switch (a.L) {
-    case 4: return launch_corr_pq<R, 1, 4>(a, S, st);
-    case 6: return launch_corr_pq<R, 2, 3>(a, S, st);
-    case 8: return launch_corr_pq<R, 1, 8>(a, S, st);
-    case 10: return launch_corr_pq<R, 2, 5>(a, S, st);
-    case 12: return launch_corr_pq<R, 3, 4>(a, S, st);
-    case 14: return launch_corr_pq<R, 2, 7>(a, S, st);
-    case 16: return launch_corr_pq<R, 4, 4>(a, S, st);
-    case 18: return launch_corr_pq<R, 3, 6>(a, S, st);
-    case 20: return launch_corr_pq<R, 4, 5>(a, S, st);
-    case 22: return launch_corr_pq<R, 2, 11>(a, S, st);
-    case 24: return launch_corr_pq<R, 3, 8>(a, S, st);
-    case 26: return launch_corr_pq<R, 2, 13>(a, S, st);
-    case 28: return launch_corr_pq<R, 4, 7>(a, S, st);
-    case 30: return launch_corr_pq<R, 5, 6>(a, S, st);
-    case 32: return launch_corr_pq<R, 4, 8>(a, S, st);
+    case 4: return launch_corr_pq<R, NF, 1, 4>(a, S, st);
+    case 6: return launch_corr_pq<R, NF, 2, 3>(a, S, st);
+    case 8: return launch_corr_pq<R, NF, 1, 8>(a, S, st);
+    case 10: return launch_corr_pq<R, NF, 2, 5>(a, S, st);
+    case 12: return launch_corr_pq<R, NF, 3, 4>(a, S, st);
+    case 14: return launch_corr_pq<R, NF, 2, 7>(a, S, st);
+    case 16: return launch_corr_pq<R, NF, 4, 4>(a, S, st);
+    case 18: return launch_corr_pq<R, NF, 3, 6>(a, S, st);
+    case 20: return launch_corr_pq<R, NF, 4, 5>(a, S, st);
+    case 22: return launch_corr_pq<R, NF, 2, 11>(a, S, st);
+    case 24: return launch_corr_pq<R, NF, 3, 8>(a, S, st);
+    case 26: return launch_corr_pq<R, NF, 2, 13>(a, S, st);
+    case 28: return launch_corr_pq<R, NF, 4, 7>(a, S, st);
+    case 30: return launch_corr_pq<R, NF, 5, 6>(a, S, st);
+    case 32: return launch_corr_pq<R, NF, 4, 8>(a, S, st);
+  }
+  if constexpr (NF == CORR_ALL && sizeof(R) == 8) {
+    switch (a.L) {
+      case 36: return launch_corr_pq<R, NF, 6, 6>(a, S, st);
+      case 40: return launch_corr_pq<R, NF, 5, 8>(a, S, st);
+    }
   }
   if constexpr (sizeof(R) == 4) {
     switch (a.L) {
-      case 36: return launch_corr_pq<R, 6, 6>(a, S, st);
-      case 40: return launch_corr_pq<R, 5, 8>(a, S, st);
-      case 42: return launch_corr_pq<R, 6, 7>(a, S, st);
-      case 48: return launch_corr_pq<R, 6, 8>(a, S, st);
+      case 36: return launch_corr_pq<R, NF, 6, 6>(a, S, st);
+      case 40: return launch_corr_pq<R, NF, 5, 8>(a, S, st);
+      case 42: return launch_corr_pq<R, NF, 6, 7>(a, S, st);
+      case 48: return launch_corr_pq<R, NF, 6, 8>(a, S, st);
     }
   }
   return QEDF_ERR_SIZE;
 }
 
+// kind 0: the sum of all four
 template <typename R>
 static int corr_entry(int kind, const R* eta, const R* g, const R* ep, const int* ps, const int* pt, int npairs,
                       int Nrv, int Lx, int Ltau, double* S, cudaStream_t st) {
-  if (kind != 1 && kind != 21 && kind != 2 && kind != 4) return QEDF_ERR_ARG;
+  if (kind != 0 && kind != 1 && kind != 21 && kind != 2 && kind != 4) return QEDF_ERR_ARG;
   if (!eta || !g || !ep || !ps || !pt || !S) return QEDF_ERR_ARG;
   if (npairs < 0 || Lx < 2 || Ltau < 1 || Nrv < 2) return QEDF_ERR_ARG;
   if ((int64_t)npairs * Ltau > INT32_MAX - 256) return QEDF_ERR_SIZE;
@@ -362,7 +420,7 @@ static int corr_entry(int kind, const R* eta, const R* g, const R* ep, const int
   a.Nt = Ltau;
   a.fa = nullptr;
   a.fb = nullptr;
-  return launch_corr<R>(a, S, st);
+  return kind == 0 ? launch_corr<R, CORR_ALL>(a, S, st) : launch_corr<R, CORR_ONE>(a, S, st);
 }
 
 }  // namespace qedf

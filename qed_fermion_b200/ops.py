@@ -194,18 +194,29 @@ def bb_corr(kind: str, eta: torch.Tensor, g_eta: torch.Tensor, ephase: torch.Ten
     all slices in one pass (fields and transforms in registers).  Returns False
     without launching on sides that the kernel is not compiled for
     (the caller then takes ``bb_pair_fields`` + FFTs + ``bb_kspace_acc``)."""
+    return _bb_corr("qedf_bb_corr", (BB_KINDS[kind],), eta, g_eta, ephase, ps, pt, Lx, S)
+
+
+def bb_corr_sum(eta: torch.Tensor, g_eta: torch.Tensor, ephase: torch.Tensor, ps: torch.Tensor, pt: torch.Tensor,
+                Lx: int, S: torch.Tensor) -> bool:
+    """:func:`bb_corr` for the sum of T1, T21, T2 and T4, whose fields share
+    their transforms: four per pair and slice instead of six."""
+    return _bb_corr("qedf_bb_corr_sum", (), eta, g_eta, ephase, ps, pt, Lx, S)
+
+
+def _bb_corr(entry, kind, eta, g_eta, ephase, ps, pt, Lx, S) -> bool:
     prec, nrv, N, Vs, Ltau = _bb_inputs("bb_corr", eta, g_eta, ephase, Lx)
     _check_cuda(ps, pt, S)
     if ps.dtype != torch.int32 or pt.dtype != torch.int32 or not ps.is_contiguous() or not pt.is_contiguous():
         raise RuntimeError("bb_corr: pair indices must be contiguous int32")
     if S.dtype != torch.complex128 or S.numel() != Vs or not S.is_contiguous() or pt.numel() != ps.numel():
         raise RuntimeError("bb_corr: S must be a contiguous complex128 buffer of Lx^2 entries")
-    st = getattr(_lib.load(), f"qedf_bb_corr_{prec}")(BB_KINDS[kind], ptr(eta), ptr(g_eta), ptr(ephase), ptr(ps), ptr(pt),
-                                            ps.numel(), nrv, Lx, Ltau, ptr(S), stream_handle())
+    st = getattr(_lib.load(), f"{entry}_{prec}")(*kind, ptr(eta), ptr(g_eta), ptr(ephase), ptr(ps), ptr(pt), ps.numel(),
+                                                nrv, Lx, Ltau, ptr(S), stream_handle())
     if st == _lib.QEDF_ERR_SIZE:
         return False
     if st != _lib.QEDF_OK:
-        raise _lib.QedfError("qedf_bb_corr", st, _lib.status_string(st))
+        raise _lib.QedfError(entry, st, _lib.status_string(st))
     _lib.LAUNCHES["count"] += 1
     return True
 

@@ -180,3 +180,35 @@ def test_one_pass_pair_sums(L, Lt, nrv, cdt):
         # each factor is a sum of L^2 terms in about 2 log2(L) + 8 roundings
         eps = torch.finfo(cdt).eps
         assert bool(((S.view(L, L) - want).abs() <= 16 * eps * np.log2(L * L) * (size + size.mean())).all()), kind
+
+
+@pytest.mark.parametrize("L,Lt,nrv,cdt", [(4, 7, 3, torch.complex64), (6, 3, 2, torch.complex128), (10, 5, 4, torch.complex64),
+                                          (20, 4, 3, torch.complex128), (22, 3, 3, torch.complex64), (26, 2, 4, torch.complex128),
+                                          (30, 5, 3, torch.complex128), (32, 2, 3, torch.complex128), (32, 3, 3, torch.complex64),
+                                          (36, 2, 3, torch.complex64), (42, 1, 3, torch.complex64), (48, 2, 3, torch.complex64),
+                                          (36, 2, 3, torch.complex128), (40, 2, 3, torch.complex128)])
+def test_one_pass_sum_of_correlators(L, Lt, nrv, cdt):
+    """The sum of T1, T21, T2 and T4 in one pass against transforms of each one's
+    fields in complex128; a pair outside the vectors counts nothing."""
+    from qed_fermion_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(L + 1)
+    eta, G = (torch.randn((nrv, Lt, L, L), dtype=cdt, device=DEV, generator=g) for _ in range(2))
+    ep = torch.exp(1j * 6.28 * torch.rand((Lt, L, L), dtype=torch.float64, device=DEV, generator=g)).to(cdt)
+    s, t = torch.combinations(torch.arange(nrv), r=2).to(torch.int32).to(DEV).T
+    ps, pt = torch.cat([s, s[:1]]).contiguous(), torch.cat([t, torch.full_like(t[:1], nrv)]).contiguous()
+    S = torch.zeros(L * L, dtype=torch.complex128, device=DEV)
+    assert ops.bb_corr_sum(eta.view(nrv, -1), G.view(nrv, -1), ep, ps, pt, L, S)
+    want, size = 0, 0
+    fields = {k: _fields_torch(k, *(x.to(torch.complex128) for x in (eta, G, ep)), s.long(), t.long())
+              for k in ("T1", "T21", "T2", "T4")}
+    trans = {k: (torch.fft.ifft2(a, norm="forward"), torch.fft.fft2(b, norm="backward")) for k, (a, b) in fields.items()}
+    for a, b in trans.values():
+        want = want + (a * b).sum(dim=(0, 1))
+    # the roundings are those of the four shared transforms: of T1's and T4's
+    # fields, at k and -k, whose half-sums T21's and T2's are
+    neg = lambda x: torch.roll(torch.flip(x, (-2, -1)), (1, 1), (-2, -1))
+    u, v = ((trans[k][0].abs(), trans[k][1].abs()) for k in ("T1", "T4"))
+    su, sv = u[0] + neg(u[1]), v[0] + neg(v[1])  # at -k
+    size = (u[0] * u[1] + v[0] * v[1] + (sv * neg(su) + neg(sv) * su) / 4).sum(dim=(0, 1))
+    eps = torch.finfo(cdt).eps
+    assert bool(((S.view(L, L) - want).abs() <= 16 * eps * np.log2(L * L) * (size + size.mean())).all())
