@@ -48,6 +48,44 @@ static int auto_segments(int64_t columns, int Nt, int blocks) {
   return best;
 }
 
+// The tile height where none is asked for; it must divide every system's L.
+// Of 2 and 4 rows the one that keeps more of the largest slices resident per
+// SM (by the warps that the kernels' 96 and 128 registers allow, up to
+// PCG_MAX_PER_SM), at equal numbers 2; 2 x 6 tiles only where neither divides
+// L.  Single precision, us per iteration with 2 x 2 and 2 x 4 tiles: L = 36, 64
+// right-hand sides, 770 and 628; L = 44, 2: 54 and 49; L = 24, 64: 202 and 224;
+// L = 48, 2: 64 and 65; 2 x 6 at L = 30, 40 right-hand sides, 338 against 282.
+static int pcg_pick_by(const PcgParams& p) {
+  int best = -1, most = 0, Lmax = 0;
+  for (int s = 0; s < p.nsys; ++s) Lmax = std::max(Lmax, p.sys[s].L);
+  for (int by : {2, 4, 6}) {
+    bool ok = true;
+    for (int s = 0; s < p.nsys; ++s) ok = ok && by_valid(p.sys[s].L, by);
+    if (!ok || (by == 6 && best > 0)) continue;
+    const int n = resident_slices(Lmax, by);
+    if (best < 0 || n > most) {
+      best = by;
+      most = n;
+    }
+  }
+  return best;
+}
+
+// 32-site elementwise units instead of 16-site ones, where none are asked for:
+// one block per SM (a wide unit's column is up to 169 KB of shared memory), two
+// rounds of narrow units and one of wide ones, whose rows are then all in flight
+// at once.  Single precision, us per iteration, 16 and 32 sites: L = 48, 2
+// right-hand sides, 53.0 and 50.8; L = 60, 1: 42.0 and 39.7; L = 66, 1: 85.7 and 81.6.
+// Three rounds against two lose (L = 52, 2: 57.6 and 59.4), and so does a wide
+// column where it takes a second block's place or L1 (L = 40, 3: 52.4 and 56.9).
+static bool wide_units(const PcgParams& p, int by, int64_t narrow, int64_t wide, int Ltau, int rhs) {
+  int Lmax = 0;
+  for (int s = 0; s < p.nsys; ++s) Lmax = std::max(Lmax, p.sys[s].L);
+  if (by <= 0) by = pcg_pick_by(p);
+  return by > 0 && resident_slices(Lmax, by) == 1 && narrow > num_sms() && wide <= num_sms() &&
+         (size_t)Ltau * 2 * PCG_CHUNK * 8 + RhsState::bytes(rhs) <= 200 * 1024;
+}
+
 int pcg_plan(PcgParams& p, const qedf_system* sys, int nsys, const qedf_pcg_opts* o) {
   std::memset(&p, 0, sizeof(p));
   if (!sys || !o || nsys <= 0 || nsys > PCG_MAX_SYS) return QEDF_ERR_ARG;
@@ -64,16 +102,24 @@ int pcg_plan(PcgParams& p, const qedf_system* sys, int nsys, const qedf_pcg_opts
   if (o->chunk == 32 && !wide_fits) return QEDF_ERR_SIZE;
   p.CH = o->chunk ? o->chunk : PCG_CHUNK;
   int Lmax = 0;
-  int64_t columns = 0, elements = 0, slices = 0;
+  int64_t columns = 0, wide = 0, elements = 0, slices = 0, all_rhs = 0;
   for (int s = 0; s < nsys; ++s) {
     const qedf_system& q = sys[s];
     if (q.Lx < 2 || q.Lx % 2 || q.Ltau < 2 || q.nrhs < 1) return QEDF_ERR_ARG;
     columns += (int64_t)q.nrhs * (((int64_t)q.Lx * q.Lx + p.CH - 1) / p.CH);
+    wide += (int64_t)q.nrhs * (((int64_t)q.Lx * q.Lx + 2 * PCG_CHUNK - 1) / (2 * PCG_CHUNK));
+    all_rhs += q.nrhs;
+    p.sys[s].L = q.Lx;
     elements += (int64_t)q.nrhs * q.Ltau * q.Lx * q.Lx;
     Lmax = std::max(Lmax, q.Lx);
     slices += (int64_t)q.nrhs * q.Ltau;
   }
   const bool may_split = elements * 2 * pcg_storage_bytes(o->mode) <= 9000000;
+  if (!o->chunk && o->mode != QEDF_PCG_PLAIN_F64 && !may_split &&
+      wide_units(p, o->by, columns, wide, ntmax_all, (int)all_rhs)) {
+    p.CH = 2 * PCG_CHUNK;
+    columns = wide;
+  }
   // blocks that take them: two per SM, or as many as the operator's slices bring
   // and fit (double precision, whose units take twice as long: L = 20, 3
   // right-hand sides, 36.9 -> 33.2 us per iteration; L = 24, 2: 35.2 -> 33.2)
@@ -325,29 +371,6 @@ int pcg_launch_kernel(const void* kern, const PcgParams& p, const BandTaps& taps
 int launch_pcg_prep(const PcgParams& p, int zero_words, cudaStream_t st) {
   k_pcg_prep<<<1, 256, 0, st>>>(p, zero_words);
   return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
-}
-
-// The tile height where none is asked for; it must divide every system's L.
-// Of 2 and 4 rows the one that keeps more of the largest slices resident per
-// SM (by the warps that the kernels' 96 and 128 registers allow, up to
-// PCG_MAX_PER_SM), at equal numbers 2; 2 x 6 tiles only where neither divides
-// L.  Single precision, us per iteration with 2 x 2 and 2 x 4 tiles: L = 36, 64
-// right-hand sides, 770 and 628; L = 44, 2: 54 and 49; L = 24, 64: 202 and 224;
-// L = 48, 2: 64 and 65; 2 x 6 at L = 30, 40 right-hand sides, 338 against 282.
-static int pcg_pick_by(const PcgParams& p) {
-  int best = -1, most = 0, Lmax = 0;
-  for (int s = 0; s < p.nsys; ++s) Lmax = std::max(Lmax, p.sys[s].L);
-  for (int by : {2, 4, 6}) {
-    bool ok = true;
-    for (int s = 0; s < p.nsys; ++s) ok = ok && by_valid(p.sys[s].L, by);
-    if (!ok || (by == 6 && best > 0)) continue;
-    const int n = resident_slices(Lmax, by);
-    if (best < 0 || n > most) {
-      best = by;
-      most = n;
-    }
-  }
-  return best;
 }
 
 int launch_pcg(PcgParams& p, int by, cudaStream_t st) {

@@ -1176,8 +1176,9 @@ static int launch_pcg_t(PcgParams& p, const BandTaps& taps, cudaStream_t st) {
     units += (int64_t)S.nrhs * S.nchunk * S.nseg;
   }
   if (eng > PcgT<RS, BY>::threads) return QEDF_ERR_SIZE;
-  // whole tau columns are the documented limit, also where they are split
-  if (sizeof(Cx<RS>) * (size_t)ntmax * p.CH > pcg_column_limit(sizeof(RS), std::max(128, eng))) return QEDF_ERR_SIZE;
+  // whole tau columns of PCG_CHUNK sites are the documented limit, also where
+  // they are split or wider
+  if (sizeof(Cx<RS>) * (size_t)ntmax * PCG_CHUNK > pcg_column_limit(sizeof(RS), std::max(128, eng))) return QEDF_ERR_SIZE;
   // the elementwise phase wants four warps; the engine's records need `eng`
   const int threads = std::max(128, eng);
   p.eng_threads = eng;
