@@ -264,13 +264,19 @@ struct TileSlot {
   __host__ __device__ static size_t smem(int threads) { return ((size_t)threads * BYTES + 15) / 16 * 16; }
 };
 
+// the engines of the operator phase and of the true residual
+template <typename RS, int BY>
+using OpSlice = Slice<RS, BY, PcgT<RS, BY>::PHS, PcgT<RS, BY>::TALL ? 1 : 2>;
+template <typename RH, int BY>
+using TrueSlice = Slice<RH, BY, true, 1>;
+
 // shared memory of the phases behind the right-hand sides' state
 template <typename RS, typename RH, typename SP, int BY>
 inline size_t pcg_phase_smem(int eng_threads, int col_rows, int CH) {
   using T = PcgT<RS, BY>;
-  size_t s = slice_smem<RS>(eng_threads, Slice<RS, BY, T::PHS, T::TALL ? 1 : 2>::REC) +
+  size_t s = slice_smem<RS>(eng_threads, OpSlice<RS, BY>::REC) +
              (T::IN_OP ? 0 : 2 * stash_smem<RS, BY>(eng_threads)) + (T::STAGE ? TileSlot<RS, BY>::smem(eng_threads) : 0);
-  if (!std::is_same<RS, RH>::value) s = std::max(s, slice_smem<RH>(eng_threads, Slice<RH, BY, true, 1>::REC));
+  if (!std::is_same<RS, RH>::value) s = std::max(s, slice_smem<RH>(eng_threads, TrueSlice<RH, BY>::REC));
   return std::max(s, sizeof(Cx<RS>) * (size_t)col_rows * CH);
 }
 
@@ -298,14 +304,14 @@ template <typename RS, typename A, typename SP, int BY>
 __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned char* smem, double& pap_out, double& ppp_out) {
   using CT = PcgT<RS, BY>;
   constexpr bool H16 = std::is_same<SP, __half>::value, LOWP = !std::is_same<SP, RS>::value;
-  using Eng = Slice<RS, BY, CT::PHS, CT::TALL ? 1 : 2>;
+  using Eng = OpSlice<RS, BY>;
   // the first two slices' angles are asked for together: at BY = 2, where
   // registers hold them, 2 to 4 % of an iteration (L = 48, 2 right-hand sides,
   // 53.6 -> 52.3 us); with taller tiles or converted storage they spill
   constexpr bool AHEAD = sizeof(RS) == 4 && BY == 2 && !LOWP;
   const int tid = threadIdx.x;
   Eng E;
-  E.init_named(q.L, smem, tid, q.eng);
+  E.init(q.L, smem, tid);
   size_t at = slice_smem<RS>(q.eng, Eng::REC);
   // y_t and y_{t+1} wait in two stashes in turn
   Stash<RS, BY> stash, other;
@@ -441,7 +447,7 @@ __device__ __forceinline__ void operator_run(const OpRun<RS, A, SP>& q, unsigned
 // ---------------------------------------------------------------------------
 template <typename RS, typename RH, typename A>
 struct TrueRun {
-  int L, Nt, a, b, eng;
+  int L, Nt, a, b;
   const A* phi;
   const RH *x, *rhs;
   RS* r;
@@ -454,8 +460,8 @@ __device__ __noinline__ double true_residual_run(const TrueRun<RS, RH, A>& q, in
   // (the address, formed here, is known to be a shared one)
   extern __shared__ __align__(128) unsigned char dsm_all[];
   unsigned char* smem = dsm_all + smem_at;
-  Slice<RH, BY, true, 1> E;
-  E.init_named(q.L, smem, threadIdx.x, q.eng);
+  TrueSlice<RH, BY> E;
+  E.init(q.L, smem, threadIdx.x);
   const int Nt = q.Nt;
   const int64_t sv = 2 * (int64_t)q.L * q.L;
   const RH t1 = (RH)q.t1, th = (RH)q.th, Cb = (RH)q.Cb;
@@ -849,6 +855,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
       }
       __syncthreads();
       if (tid < p.eng_threads) operator_run<RS, A, SP, BY>(oprun, dsm, pap, ppp);
+      else OpSlice<RS, BY>::idle_apply(1 + 2 * (b - a));
       if constexpr (H16) block_sum2_d(pap, ppp, red);
       else block_sum_d(pap, red);
       if (tid == 0) {
@@ -866,7 +873,6 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     q.Nt = S.Nt;
     q.a = a;
     q.b = b;
-    q.eng = p.eng_threads;
     q.phi = phi_all() + S.phi0 + (S.shared ? 0 : (int64_t)(v - S.rhs0) * S.Nt * 2 * S.L * S.L);
     q.x = xh() + vb;
     q.rhs = bvec() + vb;
@@ -1014,6 +1020,8 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
           if (tid < p.eng_threads) {
             const TrueRun<RS, RH, A> q = true_run(v, S, a, b);
             true_residual_run<RS, RH, A, BY, false>(q, (int)RhsState::bytes(NV));
+          } else {
+            TrueSlice<RH, BY>::idle_apply(b - a);
           }
         });
         if (!(ok = barrier())) break;
@@ -1022,6 +1030,8 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
           if (tid < p.eng_threads) {
             const TrueRun<RS, RH, A> q = true_run(v, S, a, b);
             sum = true_residual_run<RS, RH, A, BY, true>(q, (int)RhsState::bytes(NV));
+          } else {
+            TrueSlice<RH, BY>::idle_apply(b - a);
           }
           block_sum_d(sum, red);
           if (tid == 0) atomicAdd(acc.ru_rr() + v, sum);

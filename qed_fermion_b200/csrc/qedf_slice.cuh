@@ -96,8 +96,10 @@ struct Stash {
 // NBUF exchange buffers of VECS vectors per thread.  NBUF = 1 (a second
 // barrier per factor instead of a second buffer) is for kernels short of
 // shared memory.
-// A block may have more threads than its engine: init_named's barriers count the
-// engine's threads alone (whole warps).
+// A block may have more warps than its engine: those call idle_apply instead, so
+// that every barrier is the whole block's.  A barrier that counts the engine's
+// threads alone takes their number from a register: 3 to 5 % of a solver's
+// iteration (L = 48, 2 right-hand sides, 50.2 -> 48.1 us; L = 66, 1, 81.2 -> 77.1).
 // EXTRA: further entries of the record, the kernel's own.
 template <typename R, int BY, bool PHS = false, int NBUF = 2, int VECS = 1, int EXTRA = 0>
 struct Slice {
@@ -106,7 +108,6 @@ struct Slice {
   static constexpr int PH0 = NBUF * VECS * BY;  // first phase (or extra entry) of a record
   int off, rs;  // reals: this tile's first site in a slice, one row
   bool on;      // owns a tile
-  int nthr;     // threads at the engine's barriers; 0: the whole block
   Cx<R>*me, *lf, *rt, *up, *dn;  // records: own and the four neighbours'
   Cx<R> px_[PHS ? 1 : BY][2], py_[PHS ? 1 : BY][2];
 
@@ -124,17 +125,7 @@ struct Slice {
     rt = base + (on ? by * nbx + (bx + 1 == nbx ? 0 : bx + 1) : tid) * REC;
     up = base + (on ? (by == 0 ? nby - 1 : by - 1) * nbx + bx : tid) * REC;
     dn = base + (on ? (by + 1 == nby ? 0 : by + 1) * nbx + bx : tid) * REC;
-    nthr = 0;
   }
-  __device__ __forceinline__ void init_named(int L, unsigned char* smem, int tid, int threads) {
-    init(L, smem, tid);
-    nthr = threads;
-  }
-  __device__ __forceinline__ void sync() const {
-    if (nthr) asm volatile("bar.sync 1, %0;\n" ::"r"(nthr) : "memory");
-    else __syncthreads();
-  }
-
   // phase of the x-bond / y-bond starting at own site (x0+c, y0+r)
   __device__ __forceinline__ Cx<R> px(int r, int c) const {
     return PHS ? me[PH0 + 4 * r + 2 * c] : px_[PHS ? 0 : r][c];
@@ -242,7 +233,7 @@ struct Slice {
   template <int G, int BUF>
   __device__ __forceinline__ void factor(Cx<R> (&v)[BY][2]) {
     constexpr int B0 = (NBUF == 2 ? BUF : 0) * BY;
-    if constexpr (NBUF == 1) sync();  // the last factor's values are read
+    if constexpr (NBUF == 1) __syncthreads();  // the last factor's values are read
     if constexpr (G == 0 || G == 2) {
       constexpr int RC = G == 0 ? 1 : 0;  // parity of the cross rows
 #pragma unroll
@@ -252,7 +243,7 @@ struct Slice {
       }
 #pragma unroll
       for (int r = 1 - RC; r < BY; r += 2) pair(v[r][0], v[r][1], px(r, 0));
-      sync();
+      __syncthreads();
 #pragma unroll
       for (int r = RC; r < BY; r += 2) {
         v[r][1] = cfma(px(r, 1), rt[B0 + (r & ~1)], v[r][1]);
@@ -267,7 +258,7 @@ struct Slice {
       for (int r = 0; r < BY; r += 2) pair(v[r][CL], v[r + 1][CL], py(r, CL));
 #pragma unroll
       for (int r = 1; r + 1 < BY; r += 2) pair(v[r][CC], v[r + 1][CC], py(r, CC));
-      sync();
+      __syncthreads();
       v[BY - 1][CC] = cfma(py(BY - 1, CC), dn[B0], v[BY - 1][CC]);
       v[0][CC] = v[0][CC] + up[B0 + 1];
     }
@@ -284,6 +275,10 @@ struct Slice {
     factor<1, P>(v);
     factor<2, 1 - P>(v);
     factor<3, P>(v);
+  }
+  // n applications' barriers, for a warp outside the engine
+  __device__ static __forceinline__ void idle_apply(int n) {
+    for (int i = 0; i < n * 7 * (NBUF == 1 ? 2 : 1); ++i) asm volatile("bar.sync 0;\n" ::: "memory");
   }
 };
 
