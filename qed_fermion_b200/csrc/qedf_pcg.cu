@@ -49,26 +49,33 @@ static int auto_segments(int64_t columns, int Nt, int blocks) {
 }
 
 // The tile height where none is asked for; it must divide every system's L.
-// Of 2 and 4 rows the one that keeps more of the largest slices resident per
-// SM (by the warps that the kernels' 96 and 128 registers allow, up to
-// PCG_MAX_PER_SM), at equal numbers 2; 2 x 6 tiles only where neither divides
-// L.  Single precision, us per iteration with 2 x 2 and 2 x 4 tiles: L = 36, 64
-// right-hand sides, 770 and 628; L = 44, 2: 54 and 49; L = 24, 64: 202 and 224;
-// L = 48, 2: 64 and 65; 2 x 6 at L = 30, 40 right-hand sides, 338 against 282.
+// 2 x 2 tiles unless they leave an SM a single one of the largest slices and 2
+// x 4 ones more (by the warps that the kernels' 96 and 128 registers allow, up
+// to PCG_MAX_PER_SM).  Then a block's run of n slices takes 2 n + 1 B's, half
+// as many of them with two blocks per SM, each about 1.5 times as long: 2 x 2
+// where runs are so short that rounding n up and the halo eat the difference.
+// 2 x 6 tiles only where neither divides L.  us per iteration with 2 x 2 and 2 x
+// 4 tiles, mixed: L = 36, 64 right-hand sides, 741 and 614; L = 44, 5 at Ltau =
+// 308, 77 and 71; L = 44, 1 at Ltau = 440, 25.8 and 27.8 (double 63 and 86); L =
+// 48, 2, 47 and 51.  With two 2 x 2 slices per SM: L = 28, 2, 17.0 and 21.3; L =
+// 28, 6, 31.6 and 38.2 (double 85 and 108); L = 32, 4, 29.9 and 36.0; L = 28, 48,
+// 194 and 191.
 static int pcg_pick_by(const PcgParams& p) {
-  int best = -1, most = 0, Lmax = 0;
-  for (int s = 0; s < p.nsys; ++s) Lmax = std::max(Lmax, p.sys[s].L);
-  for (int by : {2, 4, 6}) {
-    bool ok = true;
-    for (int s = 0; s < p.nsys; ++s) ok = ok && by_valid(p.sys[s].L, by);
-    if (!ok || (by == 6 && best > 0)) continue;
-    const int n = resident_slices(Lmax, by);
-    if (best < 0 || n > most) {
-      best = by;
-      most = n;
-    }
+  int first = -1, Lmax = 0;
+  bool ok[7] = {};
+  int64_t slices = 0;
+  for (int s = 0; s < p.nsys; ++s) {
+    Lmax = std::max(Lmax, p.sys[s].L);
+    slices += (int64_t)p.sys[s].nrhs * p.sys[s].Nt;
   }
-  return best;
+  for (int by : {6, 4, 2}) {
+    ok[by] = true;
+    for (int s = 0; s < p.nsys; ++s) ok[by] = ok[by] && by_valid(p.sys[s].L, by);
+    if (ok[by]) first = by;
+  }
+  if (first != 2 || !ok[4] || resident_slices(Lmax, 2) > 1 || resident_slices(Lmax, 4) < 2) return first;
+  const int64_t sms = num_sms(), n2 = (slices + sms - 1) / sms, n4 = (slices + 2 * sms - 1) / (2 * sms);
+  return 3 * (2 * n4 + 1) <= 2 * (2 * n2 + 1) ? 4 : 2;
 }
 
 // 32-site elementwise units instead of 16-site ones, where none are asked for:
@@ -110,6 +117,8 @@ int pcg_plan(PcgParams& p, const qedf_system* sys, int nsys, const qedf_pcg_opts
     wide += (int64_t)q.nrhs * (((int64_t)q.Lx * q.Lx + 2 * PCG_CHUNK - 1) / (2 * PCG_CHUNK));
     all_rhs += q.nrhs;
     p.sys[s].L = q.Lx;
+    p.sys[s].Nt = q.Ltau;
+    p.sys[s].nrhs = q.nrhs;
     elements += (int64_t)q.nrhs * q.Ltau * q.Lx * q.Lx;
     Lmax = std::max(Lmax, q.Lx);
     slices += (int64_t)q.nrhs * q.Ltau;
