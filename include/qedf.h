@@ -293,9 +293,8 @@ typedef struct {
                          it is (cudaLimitPersistingL2CacheSize is never changed), released
                          to normal status after the solve by one small kernel;
                          -1: no window and no extra kernel */
-  int stage;          /* 1: the operator passes stage their input slices in shared memory by
-                         bulk copies where the stages fit (single-precision iterations);
-                         0 (default) or -1: the engine that loads them directly */
+  int stage;          /* -1, 0 or 1: accepted, has no effect (it once chose an operator
+                         engine that staged its input slices by bulk copies) */
   int x_init;         /* 1: x holds an initial guess on entry; the solve starts from the
                          residual b - A x, computed in the high precision (double for
                          MIXED / MIXED_BF16 / MIXED_F16 / PLAIN_F64).  A right-hand side with b = 0

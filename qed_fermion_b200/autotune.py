@@ -6,10 +6,9 @@ device once per problem shape and remembered:
 
 * PCG (``qedf_pcg_solve``): the tile height ``by`` of the slice engine (2, 4
   or 6 rows of the 2 x by block each thread owns), the tau-slab length of the
-  operator units (the library's load-balance search, or explicit lengths that
-  give one, two or three rounds of units per thread block), and the engine
-  that stages its input slices in shared memory against the one that loads
-  them directly, and 16- or 32-site elementwise units.
+  operator units (the library's even cut of all slices, or explicit lengths that
+  give one, two or three rounds of units per thread block), and 16- or 32-site
+  elementwise units.
 * M^dag M (``qedf_mhm_vec_*``): tile height and slab length.
 
 Each candidate runs a fixed-iteration solve of 100 iterations (or an
@@ -166,7 +165,7 @@ def pcg_choice(systems, mode, use_precon=True, dtau=0.1, iters=100, force=False,
         if hit is not None:
             return hit
     device = torch.device("cuda", torch.cuda.current_device())
-    stages = [True, False] if mode in ("mixed", "fp32", "mixed_bf16", "mixed_f16") else [False]
+    stages = [False]  # accepted by the library without effect
     chunks = [16, 32] if mode != "fp64" and max(s.Ltau for s in systems) <= 500 else [0]
     cands = [(by, T, st, ch) for by in tile_heights([s.Lx for s in systems]) for T in slab_candidates(systems)
              for st in stages for ch in chunks]

@@ -222,8 +222,6 @@ struct PcgT {
   static constexpr bool STAGE = !TALL;
   static constexpr bool PHS = IN_OP;
   static constexpr int threads = MaxT<RS, BY>::value;
-  // 80 registers at BY = 2: two 384-thread blocks per SM
-  static constexpr int min_threads = (sizeof(RS) == 4 && BY == 2) ? 768 : threads;
 };
 
 // A thread's own slot for its tile of one slice in storage type SP, filled by

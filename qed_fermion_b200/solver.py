@@ -77,10 +77,8 @@ class PcgSolver:
     (:mod:`qed_fermion_b200.autotune`), which times the candidates once per
     problem shape and caches the winner; explicit ``by`` / ``slab`` win over it.
 
-    ``stage`` lets the single-precision operator passes stage their input
-    slices in shared memory by bulk copies where the stages fit (the results
-    are the same bit for bit; measured no faster on the benchmark lattice, so
-    off by default and left to the autotuner).
+    ``stage`` is accepted and has no effect: it once chose an operator engine
+    that staged its input slices by bulk copies.
     """
 
     def __init__(self, systems: Sequence[System], mode: str = "mixed", rtol: float = 1e-10,
