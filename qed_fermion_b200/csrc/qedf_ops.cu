@@ -30,7 +30,7 @@ namespace qedf {
 // engine of qedf_slice.cuh at 8 right-hand sides, L = 48, Ltau = 480: 57 us
 // complex64 (73 with fixed slabs and one block per SM) and 187 us complex128
 // (328); the algorithmic bytes take 32 and 65 us at the copy bandwidth.  What
-// is left is issue slots (53 % busy) and shared-memory wavefronts (58 %); in
+// is left is issue slots (52 % busy) and shared-memory wavefronts (44 %); in
 // double precision the FP64 pipe, half of it for the phases' sincos.
 //
 // CFG_TALL (double precision, tall tiles with many threads): the phases live
