@@ -21,9 +21,9 @@
 // there.  Blocks per SM: at L = 30, complex128, two with 255 registers a thread
 // take 1.1 ms, three with 168 1.35 ms: the shared memory of the third is L1 that
 // the vectors' slices need.  The sum of all four, in place of T1, T21 and T4 in
-// turn: L = 30, 20 vectors, complex128 3.6 -> 1.65 ms, complex64 2.2 -> 0.95; L =
+// turn: L = 30, 20 vectors, complex128 3.6 -> 1.57 ms, complex64 2.2 -> 0.94; L =
 // 20, 1.5 -> 0.64 and 1.15 -> 0.51; L = 48, complex64, 12 vectors, 5.2 -> 1.5; L =
-// 36, complex128, 12 vectors, 4.4 -> 1.5; L = 40, 6.8 -> 2.0.
+// 36, complex128, 12 vectors, 4.4 -> 1.4; L = 40, 6.8 -> 1.8.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -190,7 +190,10 @@ struct Line {
 // fields of a pair and slice: two of one correlator, or the four of all
 constexpr int CORR_ONE = 2, CORR_ALL = 4;
 constexpr int corr_threads(int L, int NF) { return NF * L <= 128 ? 128 : (NF * L + 31) / 32 * 32; }
-constexpr int CORR_CLUSTER = 8;  // blocks that add up their sums (the portable size)
+// blocks that add up their sums; of eight, 33 clusters are resident at two blocks
+// per SM, of four all but a few SMs are filled: L = 30, complex128, 1.68 -> 1.57 ms,
+// L = 48, complex64, 1.54 -> 1.47, at the same error
+constexpr int CORR_CLUSTER = 4;
 // blocks per SM that leave a thread the registers of its line and fit in shared memory
 constexpr int corr_blocks(int L, int words, int NF) {
   if (NF == CORR_ALL && words == 1) return L <= 32 ? 4 : L <= 36 ? 3 : 2;

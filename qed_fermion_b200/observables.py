@@ -151,7 +151,7 @@ class BondBond:
     def _T_sum(self, eta, G_eta, boson):
         """T1 + T21 + T2 + T4.  One pass over the pairs where its kernel is
         compiled for the side: the four share their fields' transforms (20
-        vectors, L = 30, Ltau = 300, complex128: 3.6 -> 1.65 ms; L = 48, 12
+        vectors, L = 30, Ltau = 300, complex128: 3.6 -> 1.57 ms; L = 48, 12
         vectors, complex64: 5.2 -> 1.5)."""
         e, g, ep, pairs, S = inputs = self._pair_inputs(eta, G_eta, boson)
         dt, Vs = e.dtype, self.Lx * self.Ly
