@@ -135,7 +135,7 @@ struct PcgParams {
   void* y0;          // mixed only: half of the reliable updates' M x (the other half in Op)
   double* acc;       // accumulators
   float* ptab;       // periodic 13-band tau tables of the preconditioner, per system
-  unsigned long long* bar;  // grid barrier: arrivals (low half), error (high half)
+  unsigned long long* bar;  // grid barrier: arrivals and error (qedf_barrier_word.h)
   int* iters;
   double* relres;
   int* status;

@@ -47,6 +47,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "qedf_barrier_word.h"
 #include "qedf_internal.h"
 #include "qedf_slice.cuh"
 
@@ -55,14 +56,14 @@ namespace qedf {
 // ---------------------------------------------------------------------------
 // bounded grid barrier
 // ---------------------------------------------------------------------------
-// The low half of *bar counts arrivals over the whole solve (zeroed per solve);
+// *bar counts arrivals over the whole solve (zeroed per solve; qedf_barrier_word.h);
 // barrier n of a block is passed once the count reaches n * nblocks.  Arrival is
 // a release reduction without a reply, and waiting an acquire load of the
 // count, so the last block's arrival ends the barrier directly (release and
 // acquire at GPU scope, ordered after and before the block barriers, need no
-// further fences).  The high half is the error word: read apart, it doubled the
-// time between two looks at the count and followed the last of them.  `target` is the calling block's count to wait for, kept
-// by its thread 0 across calls.
+// further fences).  The error code is in the same word: read apart, it doubled the
+// time between two looks at the count and followed the last of them.  `target` is
+// the calling block's count to wait for, kept by its thread 0 across calls.
 __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned int nblocks, long long budget,
                                              unsigned int& target) {
   __syncthreads();
@@ -74,10 +75,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned i
     while (true) {
       unsigned long long w;
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(w) : "l"(bar) : "memory");
-      ok = (w >> 32) == 0;
-      if (!ok || (int)((unsigned int)w - target) >= 0) break;
+      ok = bar_error(w) == 0;
+      if (!ok || bar_reached(w, target)) break;
       if (clock64() - t0 > budget) {
-        atomicOr(bar, (unsigned long long)QEDF_ERR_TIMEOUT << 32);
+        atomicOr(bar, bar_error_bits(QEDF_ERR_TIMEOUT));
         ok = 0;
         break;
       }
@@ -1150,7 +1151,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     fold_pass();
   }
   if (blockIdx.x == 0) {
-    const unsigned int err = (unsigned int)(*((volatile unsigned long long*)p.bar) >> 32);
+    const unsigned int err = bar_error(*((volatile unsigned long long*)p.bar));
     for (int v = tid; v < NV; v += blockDim.x) {
       int stt = st.status()[v];
       if (err) stt = (int)err;
