@@ -145,9 +145,10 @@ struct PcgParams {
 };
 constexpr int PCG_ACC_PER_RHS = 11;
 
-// bytes that a whole tau column of an elementwise unit may have (the limit on Ltau)
+// bytes that a whole tau column of an elementwise unit may have (the limit on Ltau, 833 in double
+// precision).  Whatever the number of right-hand sides, a column within it fits beside their state.
 inline size_t pcg_column_limit(int real_bytes, int threads) {
-  return (size_t)227 * 1024 - 19 * 1024 - (real_bytes == 4 ? 128 * (size_t)threads : 0);
+  return (size_t)227 * 1024 - 19072 - (real_bytes == 4 ? 128 * (size_t)threads : 0);
 }
 
 size_t pcg_workspace_bytes(const PcgParams& p, int sloppy_bytes);

@@ -90,7 +90,7 @@ static bool wide_units(const PcgParams& p, int by, int64_t narrow, int64_t wide,
   for (int s = 0; s < p.nsys; ++s) Lmax = std::max(Lmax, p.sys[s].L);
   if (by <= 0) by = pcg_pick_by(p);
   return by > 0 && resident_slices(Lmax, by) == 1 && narrow > num_sms() && wide <= num_sms() &&
-         (size_t)Ltau * 2 * PCG_CHUNK * 8 + RhsState::bytes(rhs) <= 200 * 1024;
+         (size_t)Ltau * 2 * PCG_CHUNK * 8 + RhsState<true, true>::bytes(rhs) <= 200 * 1024;
 }
 
 int pcg_plan(PcgParams& p, const qedf_system* sys, int nsys, const qedf_pcg_opts* o) {

@@ -136,17 +136,22 @@ struct Acc {
 
 // Per-block state of the right-hand sides (identical in all blocks), carved
 // from the front of dynamic shared memory: its size follows their number, so
-// that small solves keep room for more blocks per SM.
+// that small solves keep room for more blocks per SM, and the mode, whose own
+// arrays (resmax, lastru and ru: reliable updates; scz and scp: scaled fp16) come
+// last: 71, 84 or 96 bytes each.  With all of them, 256 right-hand sides and
+// the longest tau column of double precision would not fit together.
+template <bool MIXED, bool H16>
 struct RhsState {
+  static constexpr int ND = 6 + MIXED, NI = 5 + MIXED + 3 * H16, NC = 3 + MIXED;  // doubles, ints, bytes each
   unsigned char* sm;
   int NV;
   __host__ __device__ static size_t bytes(int NV) {
-    return ((size_t)NV * (7 * 8 + 3 * 4 + 4 + 3 * 4 + 4) + 2 * (size_t)(NV + 1) * 4 + 127) / 128 * 128;
+    return ((size_t)NV * (8 * ND + 4 * NI + NC) + 2 * 4 + 127) / 128 * 128;
   }
   __device__ __forceinline__ double* d(int k) const { return reinterpret_cast<double*>(sm) + k * NV; }
-  __device__ __forceinline__ int* i(int k) const { return reinterpret_cast<int*>(d(7)) + k * NV; }
+  __device__ __forceinline__ int* i(int k) const { return reinterpret_cast<int*>(d(ND)) + k * NV; }
   __device__ __forceinline__ unsigned char* c(int k) const {
-    return reinterpret_cast<unsigned char*>(i(9) + 2) + k * NV;
+    return reinterpret_cast<unsigned char*>(i(NI) + 2) + k * NV;
   }
   __device__ __forceinline__ double* alpha() const { return d(0); }
   __device__ __forceinline__ double* beta() const { return d(1); }
@@ -154,20 +159,35 @@ struct RhsState {
   __device__ __forceinline__ double* rzold() const { return d(3); }
   __device__ __forceinline__ double* rr() const { return d(4); }
   __device__ __forceinline__ double* res() const { return d(5); }
-  __device__ __forceinline__ double* resmax() const { return d(6); }
+  __device__ __forceinline__ double* resmax() const {
+    static_assert(MIXED);
+    return d(6);
+  }
   __device__ __forceinline__ int* iters() const { return i(0); }
-  __device__ __forceinline__ int* lastru() const { return i(1); }
-  __device__ __forceinline__ int* status() const { return i(2); }
-  __device__ __forceinline__ int* list() const { return i(3); }  // a work line's right-hand sides,
-  __device__ __forceinline__ int* pre_a() const { return i(7); }  // prefix sums of their operator units
-  __device__ __forceinline__ int* pre_e() const { return i(8) + 1; }  // and of their elementwise units
+  __device__ __forceinline__ int* status() const { return i(1); }
+  __device__ __forceinline__ int* list() const { return i(2); }  // a work line's right-hand sides,
+  __device__ __forceinline__ int* pre_a() const { return i(3); }  // [NV + 1] prefix sums of their operator units
+  __device__ __forceinline__ int* pre_e() const { return i(4) + 1; }  // [NV + 1] and of their elementwise units
+  __device__ __forceinline__ int* lastru() const {
+    static_assert(MIXED);
+    return i(5) + 2;
+  }
   // storage scales of z and the two p buffers (scaled fp16)
-  __device__ __forceinline__ float* scz() const { return reinterpret_cast<float*>(i(4)); }
-  __device__ __forceinline__ float* scp(int par) const { return reinterpret_cast<float*>(i(5 + par)); }
+  __device__ __forceinline__ float* scz() const {
+    static_assert(H16);
+    return reinterpret_cast<float*>(i(5 + MIXED) + 2);
+  }
+  __device__ __forceinline__ float* scp(int par) const {
+    static_assert(H16);
+    return reinterpret_cast<float*>(i(6 + MIXED + par) + 2);
+  }
   __device__ __forceinline__ unsigned char* active() const { return c(0); }
-  __device__ __forceinline__ unsigned char* ru() const { return c(1); }
-  __device__ __forceinline__ unsigned char* pending() const { return c(2); }
-  __device__ __forceinline__ unsigned char* sys() const { return c(3); }
+  __device__ __forceinline__ unsigned char* pending() const { return c(1); }
+  __device__ __forceinline__ unsigned char* sys() const { return c(2); }
+  __device__ __forceinline__ unsigned char* ru() const {
+    static_assert(MIXED);
+    return c(3);
+  }
 };
 
 // What a block keeps about the solve, in shared memory: held in registers it
@@ -529,9 +549,10 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
   __shared__ PcgCtl ctl;
   __shared__ OpRun<RS, A, SP> oprun;
 #define NV p.nrhs
-  const RhsState st{dsm_all, NV};
+  using State = RhsState<MIXED, H16>;
+  const State st{dsm_all, NV};
   const Acc acc{p.acc, NV};
-#define dsm (dsm_all + RhsState::bytes(NV))
+#define dsm (dsm_all + State::bytes(NV))
   const int tid = threadIdx.x;
   // scales of z and of p buffer `par` (1 for every other storage type)
   auto sc_z = [&](int v) -> RS {
@@ -554,12 +575,14 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
   for (int v = tid; v < NV; v += blockDim.x) {
     st.active()[v] = 1;
     st.iters()[v] = 0;
-    st.lastru()[v] = 0;
     st.status()[v] = QEDF_OK;
     st.res()[v] = 0.0;
-    st.resmax()[v] = 1.0;
-    st.ru()[v] = 0;
     st.pending()[v] = 0;
+    if constexpr (MIXED) {
+      st.lastru()[v] = 0;
+      st.resmax()[v] = 1.0;
+      st.ru()[v] = 0;
+    }
   }
   if (tid == 0) {
     ctl.it = ctl.slot = ctl.rcur = ctl.guess = 0;
@@ -981,7 +1004,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
     __syncthreads();
     const int it = ctl.it;
     for (int v = tid; v < NV; v += blockDim.x) {
-      st.ru()[v] = 0;
+      if constexpr (MIXED) st.ru()[v] = 0;
       if (!st.active()[v]) continue;
       const double res = st.res()[v];
       if (!isfinite(res)) {
@@ -990,7 +1013,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
         ctl.changed = 1;
         continue;
       }
-      if (MIXED) {
+      if constexpr (MIXED) {
         // (the initial guess's residual is a reliable update's)
         if (res <= p.rtol || it - st.lastru()[v] >= p.ru_interval || res < p.ru_delta * st.resmax()[v] ||
             (it == 0 && p.x_init)) {
@@ -1018,7 +1041,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
         for_slices([&](int v, const PcgSys& S, int a, int b) {
           if (tid < p.eng_threads) {
             const TrueRun<RS, RH, A> q = true_run(v, S, a, b);
-            true_residual_run<RS, RH, A, BY, false>(q, (int)RhsState::bytes(NV));
+            true_residual_run<RS, RH, A, BY, false>(q, (int)State::bytes(NV));
           } else {
             TrueSlice<RH, BY>::idle_apply(b - a);
           }
@@ -1028,7 +1051,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
           double sum = 0;
           if (tid < p.eng_threads) {
             const TrueRun<RS, RH, A> q = true_run(v, S, a, b);
-            sum = true_residual_run<RS, RH, A, BY, true>(q, (int)RhsState::bytes(NV));
+            sum = true_residual_run<RS, RH, A, BY, true>(q, (int)State::bytes(NV));
           } else {
             TrueSlice<RH, BY>::idle_apply(b - a);
           }
@@ -1191,8 +1214,11 @@ static int launch_pcg_t(PcgParams& p, const BandTaps& taps, cudaStream_t st) {
   // the elementwise phase wants four warps; the engine's records need `eng`
   const int threads = std::max(128, eng);
   p.eng_threads = eng;
-  const size_t smem = RhsState::bytes(p.nrhs) + pcg_phase_smem<RS, RH, SP, BY>(eng, rows, p.CH);
-  if (smem > 226 * 1024) return QEDF_ERR_SIZE;
+  const size_t smem = RhsState<!std::is_same<RS, RH>::value, std::is_same<SP, __half>::value>::bytes(p.nrhs) +
+                      pcg_phase_smem<RS, RH, SP, BY>(eng, rows, p.CH);
+  // beside the kernel's static shared memory: red, ctl and oprun
+  constexpr size_t fixed = (64 * sizeof(double) + sizeof(PcgCtl) + sizeof(OpRun<RS, A, SP>) + 127) / 128 * 128;
+  if (smem + fixed > 227 * 1024) return QEDF_ERR_SIZE;
   auto kern = k_pcg<RS, RH, A, SP, BY>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return QEDF_ERR_CUDA;
