@@ -171,15 +171,16 @@ int qedf_bb_kspace_acc_c128(const double* A, const double* B, int64_t rows, int 
  * (ps[p], pt[p]) and all slices of A(k) B(k), A and B the unnormalised 2-D
  * transforms (e^{+2 pi i k.r / L} and e^{-2 pi i k.r / L}) of the pair's two
  * fields, which qedf_bb_pair_fields would write; the fields and transforms
- * stay on the SM.  Compiled for even Lx up to 32 and, complex64, 36, 40, 42 and
- * 48 (qedf_corr.cuh), else QEDF_ERR_SIZE: the caller then takes the two-pass
- * path. */
+ * stay on the SM.  Lx must be even and at most 32 (complex64: or 36, 40, 42, 48;
+ * qedf_corr.cuh) or split as p q with q <= 8 and fit in shared memory (complex128
+ * up to L = 48, complex64 up to L = 64; qedf_corr_any.cuh), else QEDF_ERR_SIZE:
+ * the caller then takes the two-pass path. */
 int qedf_bb_corr_c64(int kind, const float* eta, const float* g_eta, const float* ephase, const int* ps,
                      const int* pt, int npairs, int Nrv, int Lx, int Ltau, double* S, qedf_stream_t stream);
 int qedf_bb_corr_c128(int kind, const double* eta, const double* g_eta, const double* ephase, const int* ps,
                       const int* pt, int npairs, int Nrv, int Lx, int Ltau, double* S, qedf_stream_t stream);
 /* The same for the sum of T1, T21, T2 and T4, from the transforms of the four
- * fields that they share; complex128 also at Lx = 36 and 40. */
+ * fields that they share: even Lx up to 32, 36 and 40, complex64 also 42 and 48. */
 int qedf_bb_corr_sum_c64(const float* eta, const float* g_eta, const float* ephase, const int* ps, const int* pt,
                          int npairs, int Nrv, int Lx, int Ltau, double* S, qedf_stream_t stream);
 int qedf_bb_corr_sum_c128(const double* eta, const double* g_eta, const double* ephase, const int* ps, const int* pt,

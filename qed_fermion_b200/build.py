@@ -11,7 +11,7 @@ LIB = os.path.join(HERE, "libqedf.so")
 SOURCES = ["qedf_ops.cu", "qedf_pcg.cu", "qedf_pcg_f32.cu", "qedf_pcg_f64.cu", "qedf_pcg_mixed.cu", "qedf_pcg_bf16.cu",
            "qedf_pcg_f16.cu", "qedf_capi.cu", "qedf_static.cu", "qedf_bond.cu", "qedf_corr_c64.cu",
            "qedf_corr_c128.cu", "qedf_fmass.cu"]
-HEADERS = ["qedf_common.cuh", "qedf_bond.cuh", "qedf_corr.cuh", "qedf_slice.cuh", "qedf_pcg_kernel.cuh",
+HEADERS = ["qedf_common.cuh", "qedf_bond.cuh", "qedf_corr.cuh", "qedf_corr_any.cuh", "qedf_slice.cuh", "qedf_pcg_kernel.cuh",
            "qedf_barrier_word.h", "qedf_internal.h", "qedf_precon_table.h"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
          "-Xcompiler", "-fPIC", "-diag-suppress", "20013,20015"]

@@ -30,6 +30,7 @@
 #include <algorithm>
 
 #include "qedf_bond.cuh"
+#include "qedf_corr_any.cuh"
 
 namespace qedf {
 
@@ -341,6 +342,7 @@ __global__ void __launch_bounds__(corr_threads(P* Q, NF), corr_blocks(P* Q, size
 template <typename R, int NF, int P, int Q>
 static int launch_corr_pq(const BondArgs& a, double* S, cudaStream_t st) {
   constexpr int L = P * Q;
+  if (a.npairs == 0) return QEDF_OK;
   const int ni = corr_threads(L, NF) / (NF * L), threads = (ni * NF * L + 31) / 32 * 32;
   const size_t smem = L * L * sizeof(double2) + ((size_t)ni * NF * L * (L | 1) + L) * sizeof(Cx<R>);
   if (cudaFuncSetAttribute(k_bb_corr<R, P, Q, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -409,8 +411,6 @@ static int corr_entry(int kind, const R* eta, const R* g, const R* ep, const int
   if (kind != 0 && kind != 1 && kind != 21 && kind != 2 && kind != 4) return QEDF_ERR_ARG;
   if (!eta || !g || !ep || !ps || !pt || !S) return QEDF_ERR_ARG;
   if (npairs < 0 || Lx < 2 || Ltau < 1 || Nrv < 2) return QEDF_ERR_ARG;
-  if ((int64_t)npairs * Ltau > INT32_MAX - 256) return QEDF_ERR_SIZE;
-  if (npairs == 0) return QEDF_OK;
   BondArgs a;
   a.kind = kind;
   a.eta = eta;
@@ -424,7 +424,11 @@ static int corr_entry(int kind, const R* eta, const R* g, const R* ep, const int
   a.Nt = Ltau;
   a.fa = nullptr;
   a.fb = nullptr;
-  return kind == 0 ? launch_corr<R, CORR_ALL>(a, S, st) : launch_corr<R, CORR_ONE>(a, S, st);
+  // (the line kernels count items in 32 bits)
+  const bool lines = (int64_t)npairs * Ltau <= INT32_MAX - 256;
+  if (kind == 0) return lines ? launch_corr<R, CORR_ALL>(a, S, st) : QEDF_ERR_SIZE;
+  const int e = lines ? launch_corr<R, CORR_ONE>(a, S, st) : QEDF_ERR_SIZE;
+  return e == QEDF_ERR_SIZE ? launch_corr_any<R>(a, S, st) : e;
 }
 
 }  // namespace qedf

@@ -212,3 +212,31 @@ def test_one_pass_sum_of_correlators(L, Lt, nrv, cdt):
     size = (u[0] * u[1] + v[0] * v[1] + (sv * neg(su) + neg(sv) * su) / 4).sum(dim=(0, 1))
     eps = torch.finfo(cdt).eps
     assert bool(((S.view(L, L) - want).abs() <= 16 * eps * np.log2(L * L) * (size + size.mean())).all())
+
+
+@pytest.mark.parametrize("L,Lt,nrv,cdt", [(2, 9, 3, torch.complex128), (3, 7, 3, torch.complex64), (9, 4, 3, torch.complex128),
+                                          (15, 3, 4, torch.complex64), (21, 2, 3, torch.complex128), (35, 2, 3, torch.complex128),
+                                          (49, 1, 3, torch.complex64), (56, 1, 3, torch.complex64), (64, 2, 3, torch.complex64),
+                                          (36, 2, 3, torch.complex128), (42, 1, 3, torch.complex128), (48, 2, 3, torch.complex128)])
+def test_one_pass_pair_sums_on_other_sides(L, Lt, nrv, cdt):
+    """Sides that the line kernel is not compiled for and that split into factors
+    up to 8: the sum over pairs and slices against transforms of fields written
+    with torch in complex128; a pair outside the vectors counts nothing.  Odd sides
+    are the C entries' alone."""
+    from qed_fermion_b200 import _lib, ops
+    g = torch.Generator(device=DEV).manual_seed(L)
+    eta, G = (torch.randn((nrv, Lt, L, L), dtype=cdt, device=DEV, generator=g) for _ in range(2))
+    ep = torch.exp(1j * 6.28 * torch.rand((Lt, L, L), dtype=torch.float64, device=DEV, generator=g)).to(cdt)
+    s, t = torch.combinations(torch.arange(nrv), r=2).to(torch.int32).to(DEV).T
+    ps, pt = torch.cat([s, s[:1]]).contiguous(), torch.cat([t, torch.full_like(t[:1], nrv)]).contiguous()
+    for kind in ("T1", "T21", "T2", "T4"):
+        S = torch.zeros(L * L, dtype=torch.complex128, device=DEV)
+        _lib.call("qedf_bb_corr_c64" if cdt == torch.complex64 else "qedf_bb_corr_c128", ops.BB_KINDS[kind],
+                  *map(ops.ptr, (eta, G, ep, ps, pt)), len(ps), nrv, L, Lt, ops.ptr(S), ops.stream_handle())
+        a, b = _fields_torch(kind, *(x.to(torch.complex128) for x in (eta, G, ep)), s.long(), t.long())
+        prod = torch.fft.ifft2(a, norm="forward") * torch.fft.fft2(b, norm="backward")
+        want, size = prod.sum(dim=(0, 1)), prod.abs().sum(dim=(0, 1))
+        # each factor is a sum of L^2 terms in two lines of sums of at most 8 terms and a twiddle
+        # each, 40 roundings
+        eps = torch.finfo(cdt).eps
+        assert bool(((S.view(L, L) - want).abs() <= 160 * eps * (size + size.mean())).all()), kind
