@@ -15,10 +15,10 @@ one inverse FFT per observable remains; the reference instead transforms back
 per batch.  One kernel forms both fields of a pair and slice, transforms them
 and adds their product into a double-precision k-space sum (``ops.bb_corr``; for
 the sum of all four, from transforms that they share, ``ops.bb_corr_sum``).
-On sides that it is not compiled for, pairs are processed in chunks sized by
-``chunk_bytes``: per chunk one kernel writes both fields of every pair
-(``ops.bb_pair_fields``), cuFFT transforms them, and one kernel adds the
-products of the transforms to the sum (``ops.bb_kspace_acc``).
+On sides that it is not compiled for, or with ``fused=False``, pairs are
+processed in chunks sized by ``chunk_bytes``: per chunk one kernel writes both
+fields of every pair (``ops.bb_pair_fields``), cuFFT transforms them, and one
+kernel adds the products of the transforms to the sum (``ops.bb_kspace_acc``).
 
 Layouts as in the reference: eta, G_eta ``[Nrv, Ltau * Ly * Lx]`` (index
 tau Vs + x + Lx y); boson ``[1, 2, Lx, Ly, Ltau]``.  Inputs must be CUDA
@@ -32,13 +32,13 @@ from . import ops
 
 
 class BondBond:
-    def __init__(self, Lx: int, Ltau: int, chunk_bytes: int = 1 << 30, fused: bool = False):
+    def __init__(self, Lx: int, Ltau: int, chunk_bytes: int = 1 << 30, fused: bool | None = None):
         self.Lx = self.Ly = Lx
         self.Ltau = Ltau
         self.chunk_bytes = int(chunk_bytes)
-        # the pair sums take one pass (ops.bb_corr) on every lattice that kernel
-        # is compiled for, with or without ``fused``
-        self.fused = bool(fused)
+        # pair sums in one pass: on the sides where that is faster (None), on
+        # every side that one of its kernels takes (True), on none (False)
+        self.fused = fused if fused is None else bool(fused)
 
     # ---- helpers ----------------------------------------------------------
     def _chunk(self, ec, n_arrays=4):
@@ -53,7 +53,8 @@ class BondBond:
         back to real space; a_st, b_st are the fields of correlator ``kind``."""
         e, g, ep, pairs, S = inputs
         dt, nrv, Vs = e.dtype, e.shape[0], self.Lx * self.Ly
-        if ops.bb_corr(kind, e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
+        one = ops.bb_corr_lines(self.Lx, dt) if self.fused is None else self.fused
+        if one and ops.bb_corr(kind, e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
             S = S.view(self.Ly, self.Lx) / (Vs * Vs)
             return (torch.fft.ifft2(S, norm="forward") / (len(pairs) * self.Ltau)).to(dt)
         chunk = min(65535, self._chunk(e.reshape(nrv, self.Ltau, self.Ly, self.Lx)), len(pairs))
@@ -150,12 +151,13 @@ class BondBond:
 
     def _T_sum(self, eta, G_eta, boson):
         """T1 + T21 + T2 + T4.  One pass over the pairs where its kernel is
-        compiled for the side: the four share their fields' transforms (20
+        compiled for the side (and ``fused`` is not False): the four share their fields' transforms (20
         vectors, L = 30, Ltau = 300, complex128: 3.6 -> 1.57 ms; L = 48, 12
         vectors, complex64: 5.2 -> 1.5)."""
         e, g, ep, pairs, S = inputs = self._pair_inputs(eta, G_eta, boson)
         dt, Vs = e.dtype, self.Lx * self.Ly
-        if ops.bb_corr_sum(e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
+        if self.fused is not False and ops.bb_corr_sum(e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(),
+                                                       self.Lx, S):
             S = S.view(self.Ly, self.Lx) / (Vs * Vs)
             out = -(torch.fft.ifft2(S, norm="forward") / (len(pairs) * self.Ltau)).to(dt)
         else:

@@ -191,10 +191,16 @@ def bb_pair_fields(kind: str, eta: torch.Tensor, g_eta: torch.Tensor, ephase: to
 def bb_corr(kind: str, eta: torch.Tensor, g_eta: torch.Tensor, ephase: torch.Tensor, ps: torch.Tensor,
             pt: torch.Tensor, Lx: int, S: torch.Tensor) -> bool:
     """S[k] += the pair sum of correlator ``kind`` over the pairs (ps, pt) and
-    all slices in one pass (fields and transforms in registers).  Returns False
-    without launching on sides that the kernel is not compiled for
+    all slices in one pass (fields and transforms on the SM).  Returns False
+    without launching on sides that neither of its kernels takes
     (the caller then takes ``bb_pair_fields`` + FFTs + ``bb_kspace_acc``)."""
     return _bb_corr("qedf_bb_corr", (BB_KINDS[kind],), eta, g_eta, ephase, ps, pt, Lx, S)
+
+
+def bb_corr_lines(Lx: int, dtype: torch.dtype) -> bool:
+    """Whether :func:`bb_corr` takes this side with its line kernel, which beats
+    the two passes, rather than with the one for any side, which does not."""
+    return (Lx % 2 == 0 and 4 <= Lx <= 32) or (dtype == torch.complex64 and Lx in (36, 40, 42, 48))
 
 
 def bb_corr_sum(eta: torch.Tensor, g_eta: torch.Tensor, ephase: torch.Tensor, ps: torch.Tensor, pt: torch.Tensor,

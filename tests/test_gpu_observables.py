@@ -240,3 +240,50 @@ def test_one_pass_pair_sums_on_other_sides(L, Lt, nrv, cdt):
         # each, 40 roundings
         eps = torch.finfo(cdt).eps
         assert bool(((S.view(L, L) - want).abs() <= 160 * eps * (size + size.mean())).all()), kind
+
+
+@pytest.mark.parametrize("L,Lt,nrv,cdt,fused,per", [(34, 3, 4, torch.complex128, None, 4), (38, 2, 4, torch.complex64, None, 4),
+                                                    (48, 2, 3, torch.complex128, None, 2), (44, 1, 4, torch.complex64, None, 5),
+                                                    (46, 2, 4, torch.complex128, None, 1), (6, 5, 4, torch.complex64, False, 4),
+                                                    (30, 2, 3, torch.complex128, False, 2)])
+def test_two_passes_in_chunks(L, Lt, nrv, cdt, fused, per, monkeypatch):
+    """The correlators and their sum in two passes, ``per`` pairs to a chunk and a
+    ragged last one, against transforms of fields written with torch in complex128."""
+    from qed_fermion_b200 import ops
+    from qed_fermion_b200.observables import BondBond
+    g = torch.Generator(device=DEV).manual_seed(L + 2)
+    eta, G = (torch.randn((nrv, Lt, L, L), dtype=cdt, device=DEV, generator=g) for _ in range(2))
+    bos = 6.28 * torch.rand((1, 2, L, L, Lt), dtype=torch.float64, device=DEV, generator=g)
+    chunks = []
+    fields = ops.bb_pair_fields
+    monkeypatch.setattr(ops, "bb_pair_fields", lambda *a: (chunks.append(len(a[4])), fields(*a))[1])
+    bb = BondBond(L, Lt, chunk_bytes=4 * per * eta[0].numel() * eta.element_size(), fused=fused)
+    args = eta.view(nrv, -1), G.view(nrv, -1), bos
+    got = {k: getattr(bb, k)(*args) for k in ("T1", "T21", "T2_direct", "T4")}
+    n = nrv * (nrv - 1) // 2
+    assert chunks == 4 * ([per] * (n // per) + [n % per] * (n % per > 0))  # all four in two passes
+    chunks.clear()
+    got["sum"] = bb.get_bond_bond_per_b2(*args)["BB0_r"] / 2
+    assert sum(chunks) == 3 * n
+
+    e, G, ep = (x.to(torch.complex128) for x in (eta, G, torch.exp(1j * bos[0, 0].permute(2, 1, 0))))
+    s, t = torch.combinations(torch.arange(nrv, device=DEV), r=2).T
+    at = lambda x, k: torch.roll(x, -k, -1)  # x at r + k
+    short = {"T1": ((0, -1), at(G, 1) * at(e, -1).conj() * ep * at(ep, -1)), "T21": ((0, 0), G * e.conj()),
+             "T4": ((0, 1), G * at(e, 2).conj() * (ep * at(ep, 1)).conj())}
+    short["T2_direct"] = short["T21"]
+    want, tol = {"sum": 0}, {"sum": 0}
+    eps = torch.finfo(cdt).eps
+    for k, (d, terms) in short.items():
+        a, b = _fields_torch(k[:2] if k == "T2_direct" else k, e, G, ep, s, t)
+        prod = torch.fft.ifft2(a) * torch.fft.fft2(b) / (n * Lt * L * L)
+        want[k] = -torch.fft.ifft2(prod.sum(dim=(0, 1)), norm="forward")
+        want[k][d] += terms.mean()
+        # a transform's error per k is below 8 eps log2(L^2) of its size (cuFFT's and the fields'
+        # roundings), of the product twice that, and a sum over k adds them all; then the
+        # short-distance terms' products, the results' rounding and the reference's own
+        tol[k] = 32 * eps * np.log2(L * L) * prod.abs().sum() + 8 * eps * (terms.abs().mean() + want[k].abs())
+        want["sum"], tol["sum"] = want["sum"] + want[k], tol["sum"] + tol[k]
+    want["sum"] = want["sum"].real
+    for k in got:
+        assert bool(((got[k] - want[k]).abs() <= tol[k]).all()), k
