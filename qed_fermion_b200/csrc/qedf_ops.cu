@@ -7,6 +7,7 @@
 //   forces   same as angles
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 
 #include "qedf_internal.h"
 #include "qedf_slice.cuh"
@@ -221,13 +222,16 @@ __global__ void __launch_bounds__(MaxT<R, BY>::value, 1) k_bvec(BvecArgs p) {
 // A warp forms C consecutive output rows of 32 sites; a block's warps take
 // neighbouring segments of tau, whose common rows meet in L1.  The C + 2H rows
 // of r that a banded P_tau needs are all loaded at once, into registers, while
-// the warp finds out which rows of its segment are the middle CSR row (t =
-// Ltau/2) shifted along tau - taps t-H .. t+H with the same values, as in the
-// bulk.  Those rows then need registers only, with the taps as constants.  The
-// others, a few at the ends of tau, are dealt to all warps of the block, which
-// run over the CSR row: a lane holds an entry, the warp reads eight rows of r
-// at a time.  Both orders of summation are the CSR order, so the two forms
-// agree bit for bit.  What is left is loads in flight against the 60 MB of the
+// the warp finds out which of three forms each row of its segment has:
+// * the middle CSR row (t = Ltau/2) shifted along tau - taps t-H .. t+H with the
+//   same values, as in the bulk: registers only, with the taps as constants;
+// * up to 2H+1 entries within t-H .. t+H in ascending order: registers too, with
+//   the row's own taps from shared memory, absent ones left out;
+// * any other: dealt to all warps of the block, which run over the CSR row 32
+//   entries at a time, the next ones on their way; from shared memory an
+//   entry is one broadcast where shuffles took two or three.
+// All orders of summation are the CSR order, so the forms agree bit for bit.
+// What is left is loads in flight against the 60 MB of the
 // first size below.  Measured against columns staged in shared memory: 8
 // vectors at L = 36, Ltau = 359, complex64, 29.5 -> 21 us (complex128 52 -> 37);
 // 8 at 48 / 480, 54 -> 43 us.  With the rows of r asked for before the entries,
@@ -239,6 +243,10 @@ template <>
 struct Tap<float> {
   static constexpr int ROWS = 16;
   using V = float2;
+  struct __align__(8) Entry {
+    float v;
+    int c;
+  };
   unsigned long long c;  // the tap twice: one instruction for both parts
   __device__ __forceinline__ explicit Tap(float t) { asm("mov.b64 %0, {%1, %1};" : "=l"(c) : "f"(t)); }
   __device__ __forceinline__ V fma(V q, V a) const {
@@ -251,6 +259,10 @@ template <>
 struct Tap<double> {
   static constexpr int ROWS = 8;
   using V = double2;
+  struct __align__(16) Entry {
+    double v;
+    int c;
+  };
   double c;
   __device__ __forceinline__ explicit Tap(double t) : c(t) {}
   __device__ __forceinline__ V fma(V q, V a) const { return make_double2(::fma(c, q.x, a.x), ::fma(c, q.y, a.y)); }
@@ -264,7 +276,10 @@ __global__ void __launch_bounds__(32 * PRE_WARPS, 4) k_precon(PreconArgs p) {
   using V = typename Tap<R>::V;
   constexpr int H = PRE_H, C = Tap<R>::ROWS, TAPS = 2 * H + 1;
   constexpr unsigned ALL = 0xffffffffu;
-  __shared__ unsigned odd[PRE_WARPS];  // rows that are not the middle one
+  using Entry = typename Tap<R>::Entry;
+  __shared__ unsigned odd[PRE_WARPS];  // rows of the last form
+  __shared__ R taps[PRE_WARPS][C][TAPS];  // of rows of the second form
+  __shared__ __align__(16) Entry entries[PRE_WARPS][2][32];
   const int Vs = p.L * p.L, Nt = p.Nt, nchunk = (Vs + 31) / 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t rb = blockIdx.x / nchunk;
@@ -318,7 +333,51 @@ __global__ void __launch_bounds__(32 * PRE_WARPS, 4) k_precon(PreconArgs p) {
     if (t0 < H) mask &= ALL << (H - t0);
     if (t0 + C > Nt - H) mask &= t0 < Nt - H ? (1u << (Nt - H - t0)) - 1 : 0u;
   }
-  if (lane == 0) odd[w] = ~mask & ((1u << rows) - 1);
+  // rows whose own taps lie within H slices
+  const unsigned rest = ~mask & ((1u << rows) - 1);
+  unsigned near = 0, have = 0;
+  if (rest) {
+    constexpr int PARTS = 32 / C, PER = (TAPS + PARTS - 1) / PARTS;  // lanes to a row, entries to a lane
+    const int g = lane % C, part = lane / C;
+    const int kg = __shfl_sync(ALL, kl, g), ng = __shfl_sync(ALL, kl, g + 1) - kg;
+    bool ok = (rest >> g & 1) && ng <= TAPS;
+    int off[PER];
+    double v[PER];
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+      const int i = part * PER + n;
+      off[n] = -1;
+      if (ok && i < ng) {
+        off[n] = p.col[kg + i];
+        v[n] = p.val[kg + i];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+      if (!ok || part * PER + n >= ng) continue;
+      const bool in = (unsigned)off[n] < (unsigned)Nt;
+      off[n] -= t0 + g - H;
+      ok = in && (unsigned)off[n] < (unsigned)TAPS;
+      if (!ok) continue;
+      have |= 1u << off[n];
+      taps[w][g][off[n]] = (R)v[n];
+    }
+#pragma unroll
+    for (int o = C; o < 32; o *= 2) have |= __shfl_xor_sync(ALL, have, o);
+    // ascending: as many of the row's entries lie below each as precede it
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+      const int i = part * PER + n;
+      if (ok && i < ng) ok = __popc(have & ((1u << off[n]) - 1)) == i;
+    }
+    ok = ok && __popc(have) == ng;
+    near = __ballot_sync(ALL, ok);
+#pragma unroll
+    for (int o = C; o < 32; o *= 2) near &= near >> o;
+    near &= rest;
+    __syncwarp();
+  }
+  if (lane == 0) odd[w] = rest & ~near;
   if (mask) {
     const R vr = (R)vm;
     R c[TAPS];
@@ -334,33 +393,96 @@ __global__ void __launch_bounds__(32 * PRE_WARPS, 4) k_precon(PreconArgs p) {
       if (on) __stcg(z0 + (int64_t)i * Vs, acc);
     }
   }
-  __syncthreads();
-  int at = 0;  // odd rows before this one in the block
-  for (int g = 0; g < PRE_WARPS; ++g)
-    for (unsigned m = odd[g]; m; m &= m - 1, ++at) {
-      if (at % PRE_WARPS != w) continue;
-      const int t = b0 + g * C + __ffs(m) - 1, k1 = p.row_ptr[t + 1];
+  if (near) {
+    V* z0 = z + (int64_t)t0 * Vs;
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const unsigned h = __shfl_sync(ALL, have, i);
+      if (!(near >> i & 1)) continue;
       V acc = {0, 0};
-      for (int k = p.row_ptr[t]; k < k1; k += 32) {
-        const int cl = k + lane < k1 ? p.col[k + lane] : -1;
-        const R vl = k + lane < k1 ? (R)p.val[k + lane] : R(0);
-        for (int e = 0; e < min(32, k1 - k); e += 8) {
-          V qe[8];
-          int cc[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            cc[i] = __shfl_sync(ALL, cl, e + i);
-            qe[i] = r[(int64_t)min((unsigned)cc[i], (unsigned)Nt - 1) * Vs];
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const V next = Tap<R>(__shfl_sync(ALL, vl, e + i)).fma(qe[i], acc);
-            if ((unsigned)cc[i] < (unsigned)Nt) acc = next;  // else: outside the matrix
-          }
-        }
-      }
-      if (on) __stcg(z + (int64_t)t * Vs, acc);
+      for (int k = 0; k < TAPS; ++k)
+        if (h >> k & 1) acc = Tap<R>(taps[w][i][k]).fma(q[i + k], acc);
+      if (on) __stcg(z0 + (int64_t)i * Vs, acc);
     }
+  }
+  __syncthreads();
+  // this warp's rows of the last form, one per lane: the block's w-th, (w + PRE_WARPS)-th ...
+  int mine = -1, left = w + PRE_WARPS * lane;
+#pragma unroll
+  for (int g = 0; g < PRE_WARPS; ++g) {
+    unsigned m = odd[g];
+    const int n = __popc(m);
+    if (mine < 0 && left < n) {
+      for (int k = 0; k < left; ++k) m &= m - 1;
+      mine = g * C + __ffs(m) - 1;
+    }
+    left -= n;
+  }
+  const int own = __popc(__ballot_sync(ALL, mine >= 0));  // (at most C)
+  if (!own) return;
+  int first = 0, end = 0;
+  if (mine >= 0) {
+    first = p.row_ptr[b0 + mine];
+    end = p.row_ptr[b0 + mine + 1];
+  }
+  int cl = -1, buf = 0;
+  R vl = 0;
+  auto ask = [&](int k, int k1) {  // entries k .. k + 31 below k1
+    cl = -1;
+    if (k + lane < k1) {
+      cl = p.col[k + lane];
+      vl = (R)p.val[k + lane];
+    }
+  };
+  ask(__shfl_sync(ALL, first, 0), __shfl_sync(ALL, end, 0));
+  for (int j = 0; j < own; ++j) {
+    int k = __shfl_sync(ALL, first, j);
+    const int k1 = __shfl_sync(ALL, end, j), t = b0 + __shfl_sync(ALL, mine, j);
+    const int kn = __shfl_sync(ALL, first, min(j + 1, own - 1)), kn1 = j + 1 < own ? __shfl_sync(ALL, end, j + 1) : 0;
+    V acc = {0, 0};
+    do {
+      // (two buffers: the one before this is read by all once they meet here)
+      entries[w][buf][lane] = {vl, cl};
+      // (a lane without an entry has column -1)
+      const bool inside = __all_sync(ALL, (unsigned)cl < (unsigned)Nt || k + lane >= k1);
+      __syncwarp();
+      constexpr int N = 16 / sizeof(Entry);  // entries to an access
+      struct __align__(16) Entries {
+        Entry e[N];
+      };
+      const Entries* en = reinterpret_cast<const Entries*>(entries[w][buf]);
+      buf ^= 1;
+      const int n = min(32, k1 - k);
+      k += 32;
+      if (k < k1) ask(k, k1);
+      else ask(kn, kn1);
+      auto add = [&](auto count, auto check, int e) {  // entries e .. e + count - 1
+        constexpr int M = decltype(count)::value;
+        constexpr bool CHECK = decltype(check)::value;
+        V qe[M];
+        Entries x[M / N];
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+          if (i % N == 0) x[i / N] = en[(e + i) / N];
+          const unsigned c = x[i / N].e[i % N].c;
+          qe[i] = r[(int64_t)(CHECK ? min(c, (unsigned)Nt - 1) : c) * Vs];
+        }
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+          const Entry& q = x[i / N].e[i % N];
+          const V next = Tap<R>(q.v).fma(qe[i], acc);
+          if (!CHECK || (unsigned)q.c < (unsigned)Nt) acc = next;  // else: outside the matrix
+        }
+      };
+      int e = 0;
+      if (inside)
+        for (; n - e >= 8; e += 8) add(std::integral_constant<int, 8>(), std::false_type(), e);
+      for (; n - e > 4; e += 8) add(std::integral_constant<int, 8>(), std::true_type(), e);
+      if (e < n) add(std::integral_constant<int, 4>(), std::true_type(), e);
+    } while (k < k1);
+    if (on) __stcg(z + (int64_t)t * Vs, acc);
+  }
 }
 
 // ============================================================================
