@@ -1027,6 +1027,33 @@ int pick_by(int L, int requested, int real_bytes) {
   return best;
 }
 
+// slices that the busiest block place of the GPU gets, `resident` slices to an SM
+static int64_t rounds_of(int64_t slices, int resident) {
+  const int64_t places = (int64_t)num_sms() * resident;
+  return (slices + places - 1) / places;
+}
+
+// The operators' tile height.  In single precision 2 x 2 tiles in place of 2 x 6 ones
+// where the slices would fill half of the block places of 2 x 2 tiles at most: a slice's
+// own time counts there (L = 18, M^dag M, us with 2 x 2 and 2 x 6 tiles: 1 vector 3.8
+// and 5.5, 4: 4.7 and 5.7, 8: 7.0 and 6.8).  In double precision 2 x 4 tiles, where
+// pick_by prefers them, have to shorten the busiest block's run: a run of n slices
+// applies B n times and starts up once, M^dag M 2 n + 1 times, each the longer
+// the more slices share the SM.  Measured with 2 x 2 and 2 x 4 tiles, us:
+// M^dag M at L = 28, 2 vectors, 16.9 and 20.9, 8: 45.6 and 45.5; L = 32, 3: 30.7 and
+// 29.1, 8: 55.9 and 51.6; L = 36, 1: 20.9 and 23.3, 8: 98.8 and 84.9; L = 20, 2: 10.8
+// and 12.7, 8: 26.9 and 20.9; M at L = 36, 1: 14.7 and 16.6, 3: 31.1 and 27.1.
+static int pick_operator_by(int op, const OpArgs& a, int requested, int real_bytes) {
+  const int by = pick_by(a.L, requested, real_bytes);
+  if (requested > 0 || !by_valid(a.L, 2)) return by;
+  const int64_t W = (int64_t)a.bs * a.Nt;
+  const int r2 = resident_slices(a.L, 2, real_bytes), r4 = resident_slices(a.L, 4, real_bytes);
+  if (real_bytes == 4) return by == 6 && rounds_of(2 * W, r2) == 1 ? 2 : by;
+  if (by != 4) return by;
+  auto cost = [&](int r) { return op == OP_MHM ? 2 * rounds_of(W, r) + 1 : rounds_of(W, r) + 1; };
+  return (r2 + r4) * cost(r4) < 2 * r2 * cost(r2) ? 4 : 2;
+}
+
 static size_t smem_limit() { return 227 * 1024; }
 
 // blocks of a run-per-block kernel: as many as the GPU holds at once, but
@@ -1086,7 +1113,7 @@ static int launch_operator_by(int op, const OpArgs& a, cudaStream_t st) {
 
 template <typename R, typename A>
 int launch_operator(int op, OpArgs a, int by, cudaStream_t st) {
-  by = pick_by(a.L, by, sizeof(R));
+  by = pick_operator_by(op, a, by, sizeof(R));
   switch (by) {
     case 2: return launch_operator_by<R, A, 2>(op, a, st);
     case 4: return launch_operator_by<R, A, 4>(op, a, st);
