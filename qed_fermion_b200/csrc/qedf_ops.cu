@@ -1170,9 +1170,27 @@ static int launch_force_by(const ForceArgs& a, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? QEDF_OK : QEDF_ERR_CUDA;
 }
 
+// The force's tile height.  Its kernels keep 112, 128 and 168 registers (18, 16
+// and 12 warps per SM), and where 2 x 2 tiles leave an SM two slices or more (in
+// double precision one), the taller tile that pick_by prefers has to cut the rounds
+// of slices by more than each one's longer time: 1.7 times with 2 x 4 and twice with 2 x
+// 6 tiles in single, 1.95 times with 2 x 4 in double precision.  Measured with 2 x 2 and
+// the taller tiles, us: complex64, L = 30, 2 vectors, 14.6 and 17.3 (2 x 6), 8: 33.4 and
+// 39.0; L = 18, 8: 12.7 and 10.5; L = 32, 2: 13.4 and 15.0 (2 x 4), 8: 33.4 and 31.5;
+// complex128, L = 32, 1: 19.0 and 17.0, 2: 27.3 and 33.5; L = 36, 1: 23.1 and 29.3, 8:
+// 136 and 134.
+static int pick_force_by(const ForceArgs& a, int requested, int real_bytes) {
+  const int by = pick_by(a.L, requested, real_bytes);
+  if (requested > 0 || by <= 2 || !by_valid(a.L, 2)) return by;
+  auto slices = [&](int h) { return (h == 2 ? 18 : h == 4 ? 16 : 12) / (slice_threads(a.L, h) / 32); };
+  auto rounds = [&](int h) { return rounds_of((int64_t)a.bs * a.Nt, slices(h)); };
+  if (slices(by) < 1 || (real_bytes == 4 && slices(2) < 2)) return by;
+  return (real_bytes == 8 ? 1.95 : by == 4 ? 1.7 : 2.0) * rounds(by) <= rounds(2) ? by : 2;
+}
+
 template <typename R, typename A>
 int launch_force(ForceArgs a, int by, cudaStream_t st) {
-  by = pick_by(a.L, by, sizeof(R));
+  by = pick_force_by(a, by, sizeof(R));
   switch (by) {
     case 2: return launch_force_by<R, A, 2>(a, st);
     case 4: return launch_force_by<R, A, 4>(a, st);
