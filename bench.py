@@ -498,7 +498,7 @@ def run_native(args):
         e1.record(stream)
         torch.cuda.synchronize()
         t = e0.elapsed_time(e1) / 1e3
-        shape = ({k: h.solver.tuned[k] for k in ("by", "slab", "stage", "chunk")} if h.solver.tuned else None)
+        shape = ({k: h.solver.tuned[k] for k in ("by", "slab", "chunk")} if h.solver.tuned else None)
         return {"value": 3600.0 * n * bs / t, "unit": UNIT, "steps": n, "s_per_trajectory": t / n,
                 "cg_iters_per_solve": float(torch.stack(its).double().mean()), "pcg_launch_shape": shape}
 
@@ -697,7 +697,7 @@ def run_native(args):
             "fp64_plain": fp64, "speedup_vs_fp64": (value / world) / fp64["value"] if fp64 else None,
             "speedup_vs_fp64_dropin": ((value / world) / fp64["dropin"]["value"]
                                        if fp64 and "dropin" in fp64 else None),
-            "pcg_launch_shape": ({k: hmc.solver.tuned[k] for k in ("by", "slab", "stage", "chunk")}
+            "pcg_launch_shape": ({k: hmc.solver.tuned[k] for k in ("by", "slab", "chunk")}
                                  if hmc.solver.tuned else None),
             "bf16": bf16, "f16": f16, "all_options": fastest, "graph": graph, "chrono": chrono, "delta_H": dH, "mhm_matvec": mhm, "acceptance": acc_rate,
             "acceptance_vs_fp64": acc, **result,
@@ -893,7 +893,7 @@ def run_configs(args):
 
     def tuned(solver):
         t = solver.tuned
-        return None if t is None else {k: t[k] for k in ("by", "slab", "stage", "chunk", "us_per_iter")}
+        return None if t is None else {k: t[k] for k in ("by", "slab", "chunk", "us_per_iter")}
 
     # C2: uniform angles, b = M^dag eta
     L, Lt = 24, 240

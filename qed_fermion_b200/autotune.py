@@ -153,8 +153,8 @@ def _synthetic(systems, angle_dtype, vec_dtype, device, seed=20261204):
 
 
 def pcg_choice(systems, mode, use_precon=True, dtau=0.1, iters=100, force=False, warm_seconds=1.0) -> dict:
-    """The fastest (by, slab, stage) for this batch of systems and precision
-    mode, timed once and then cached.  Returns a dict with the choice, its
+    """The fastest (by, slab, chunk) for this batch of systems and precision
+    mode, timed once and then cached ("stage": an option without effect).  Returns a dict with the choice, its
     microseconds per iteration and the timings of every candidate."""
     from .solver import PcgSolver
     shape = {"systems": [[s.Lx, s.Ltau, s.nrhs, int(s.shared_boson)] for s in systems], "mode": mode,
@@ -165,16 +165,15 @@ def pcg_choice(systems, mode, use_precon=True, dtau=0.1, iters=100, force=False,
         if hit is not None:
             return hit
     device = torch.device("cuda", torch.cuda.current_device())
-    stages = [False]  # accepted by the library without effect
     chunks = [16, 32] if mode != "fp64" and max(s.Ltau for s in systems) <= 500 else [0]
-    cands = [(by, T, st, ch) for by in tile_heights([s.Lx for s in systems]) for T in slab_candidates(systems)
-             for st in stages for ch in chunks]
+    cands = [(by, T, ch) for by in tile_heights([s.Lx for s in systems]) for T in slab_candidates(systems)
+             for ch in chunks]
     phi = b = None
     timings = []
-    for by, T, st, ch in cands:
+    for by, T, ch in cands:
         try:
             s = PcgSolver(systems, mode=mode, rtol=0.0, max_iter=iters, dtau=dtau, use_precon=use_precon,
-                          by=by, slab=T, stage=st, chunk=ch, device=device, tune=False)
+                          by=by, slab=T, chunk=ch, device=device, tune=False)
         except (ValueError, _lib.QedfError):
             continue
         if phi is None:
@@ -188,7 +187,7 @@ def pcg_choice(systems, mode, use_precon=True, dtau=0.1, iters=100, force=False,
             ms = _time(lambda: s.solve(phi, b), reps=3)
         except _lib.QedfError:
             continue  # a shape this launch cannot take (shared memory, threads)
-        timings.append({"by": by, "slab": T, "stage": st, "chunk": ch, "us_per_iter": 1e3 * ms / iters})
+        timings.append({"by": by, "slab": T, "stage": False, "chunk": ch, "us_per_iter": 1e3 * ms / iters})
         del s
     if not timings:
         # no launch shape takes this batch (e.g. a lattice beyond the slice
@@ -198,7 +197,7 @@ def pcg_choice(systems, mode, use_precon=True, dtau=0.1, iters=100, force=False,
         _remember(key, out)
         return out
     best = min(timings, key=lambda t: t["us_per_iter"])
-    out = {"by": best["by"], "slab": best["slab"], "stage": best["stage"], "chunk": best["chunk"],
+    out = {"by": best["by"], "slab": best["slab"], "stage": False, "chunk": best["chunk"],
            "us_per_iter": best["us_per_iter"], "candidates": timings}
     _remember(key, out)
     return out

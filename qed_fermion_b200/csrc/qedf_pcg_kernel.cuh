@@ -17,7 +17,7 @@
 // The last iteration's x update is applied by a reliable update's fold or at
 // the end of the solve.
 //
-// which is the arithmetic of preconditioned_cg_fast_test
+// This is the arithmetic of preconditioned_cg_fast_test
 // (hmc_sampler_batch.py:751-846) with the reference's per-iteration torch
 // kernels (einsum dots, axpys, _C.mhm_vec, _C.precon_vec) fused.  Every
 // right-hand side has its own mask: once ||r||/||b|| <= rtol it stops
@@ -245,28 +245,17 @@ struct PcgT {
   static constexpr int threads = MaxT<RS, BY>::value;
 };
 
-// A thread's own slot for its tile of one slice in storage type SP, filled by
-// cp.async (each thread waits for its own copies only).
-template <typename SP, int BY, int STRIDE = 0>
+// A thread's own slot for its tile of one slice, filled by cp.async with an L2
+// evict-first policy (each thread waits for its own copies only).
+template <typename SP, int BY>
 struct TileSlot {
-  static constexpr int ROW = 4 * sizeof(SP);  // bytes of two complex numbers: 8, 16 or 32
+  static constexpr int ROW = 4 * sizeof(SP);  // bytes of two complex numbers or four angles: 16 or 32
   // odd multiples of the access width apart
-  static constexpr int BYTES = STRIDE ? STRIDE : ROW == 8 ? 8 * (BY | 1) : 16 * ((ROW / 16 * BY) | 1);
+  static constexpr int BYTES = 16 * ((ROW / 16 * BY) | 1);
   unsigned char* p;
   __device__ __forceinline__ void init(unsigned char* smem, int tid) { p = smem + (size_t)tid * BYTES; }
   __device__ __forceinline__ SP* row(int r) const { return reinterpret_cast<SP*>(p + r * ROW); }
   // src: the tile's first site, rs: reals per row of the slice
-  __device__ __forceinline__ void fetch(const SP* src, int rs) const {
-#pragma unroll
-    for (int r = 0; r < BY; ++r) {
-      if constexpr (ROW == 8) {
-        cp_async8(row(r), src + r * rs);
-      } else {
-#pragma unroll
-        for (int k = 0; k < ROW / 16; ++k) cp_async16(row(r) + 16 / sizeof(SP) * k, src + r * rs + 16 / sizeof(SP) * k);
-      }
-    }
-  }
   __device__ __forceinline__ void fetch_first(const SP* src, int rs) const {
     const unsigned long long pol = evict_first_policy();
 #pragma unroll
@@ -274,11 +263,6 @@ struct TileSlot {
 #pragma unroll
       for (int k = 0; k < ROW / 16; ++k)
         cp_async16(row(r) + 16 / sizeof(SP) * k, src + r * rs + 16 / sizeof(SP) * k, pol);
-  }
-  template <typename R>
-  __device__ __forceinline__ void take(Cx<R> (&v)[BY][2], R sc) const {
-#pragma unroll
-    for (int r = 0; r < BY; ++r) ld2s(row(r), v[r][0], v[r][1], sc);
   }
   __host__ __device__ static size_t smem(int threads) { return ((size_t)threads * BYTES + 15) / 16 * 16; }
 };
@@ -839,7 +823,7 @@ __global__ void __launch_bounds__(PcgT<RS, BY>::threads, 1)
   };
 
   // ---- operator pass over this block's runs of slices ------------------------------
-    auto operator_pass = [&](int slot) {
+  auto operator_pass = [&](int slot) {
     for_slices([&](int v, const PcgSys& S, int a, int b) {
       double pap = 0, ppp = 0;
       __syncthreads();

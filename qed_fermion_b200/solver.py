@@ -73,7 +73,7 @@ class PcgSolver:
     set-aside as it is (the limit is never changed), and releases the window's
     lines after the solve.  Pass False for no window.
 
-    ``tune`` takes ``by``, ``slab`` and ``stage`` from the autotuner
+    ``tune`` takes ``by``, ``slab`` and ``chunk`` from the autotuner
     (:mod:`qed_fermion_b200.autotune`), which times the candidates once per
     problem shape and caches the winner; explicit ``by`` / ``slab`` win over it.
 
@@ -97,7 +97,7 @@ class PcgSolver:
             from . import autotune
             with torch.cuda.device(self.device):
                 self.tuned = autotune.pcg_choice(self.systems, mode, use_precon=use_precon, dtau=dtau)
-            by, slab, stage = self.tuned["by"], self.tuned["slab"], self.tuned["stage"]
+            by, slab = self.tuned["by"], self.tuned["slab"]
             chunk = self.tuned.get("chunk", chunk)
         n = len(self.systems)
         self._sys = (_lib.QedfSystem * n)(*[_lib.QedfSystem(s.Lx, s.Ltau, s.nrhs, 1 if s.shared_boson else 0)
