@@ -36,7 +36,7 @@ UNIT = "trajectories/hour"
 # DRAM bytes (read + write) per site and PCG iteration of k_pcg on this
 # workload, mixed precision, 2 right-hand sides: ncu --metrics
 # dram__bytes_read.sum,dram__bytes_write.sum of `bench.py --solve-only 482`
-PCG_DRAM_BYTES_PER_SITE_ITER = 72.7
+PCG_DRAM_BYTES_PER_SITE_ITER = 59.4
 # PCG iterations per solve of this workload (mixed, rtol 1e-10) as the GPU run
 # measures them: the CPU arms' fallback when they run neither a GPU solve nor
 # their own trajectory
@@ -931,7 +931,7 @@ def run_configs(args):
     del se16
     ms, _ = timed(lambda: se.get_bond_bond_per_b2(bos))
     emit({"config": "C4a", "what": "bond-bond correlators T1+T21+T2+T4+Tvv over the 2016 noise pairs "
-                                   "(complex128, pair-field and k-space kernels around cuFFT)", "ms": ms})
+                                   "(complex128, one pass for the sum of the four)", "ms": ms})
     se.corr_dtype = torch.complex64
     ms, _ = timed(lambda: se.get_bond_bond_per_b2(bos))
     emit({"config": "C4a", "what": "the same correlators in complex64 (the reference estimator's precision)",
