@@ -28,8 +28,8 @@ namespace qedf {
 // The slices of all right-hand sides form one line that is cut into one
 // contiguous run per block (block_run), so every SM gets the same number of
 // slices; with a slab length, a run is one slab instead.  Measured with the
-// engine of qedf_slice.cuh at 8 right-hand sides, L = 48, Ltau = 480: 57 us
-// complex64 (73 with fixed slabs and one block per SM) and 187 us complex128
+// engine of qedf_slice.cuh at 8 right-hand sides, L = 48, Ltau = 480: 60 us
+// complex64 (72 with fixed slabs and one block per SM) and 191 us complex128
 // (328); the algorithmic bytes take 32 and 65 us at the copy bandwidth.  What
 // is left is issue slots (52 % busy) and shared-memory wavefronts (44 %); in
 // double precision the FP64 pipe, half of it for the phases' sincos.
@@ -247,12 +247,15 @@ __global__ void __launch_bounds__(MaxT<R, BY>::value, 1) k_bvec(BvecArgs p) {
 //   entries at a time, the next ones on their way; from shared memory an
 //   entry is one broadcast where shuffles took two or three.
 // All orders of summation are the CSR order, so the forms agree bit for bit.
-// What is left is loads in flight against the 60 MB of the
-// first size below.  Measured against columns staged in shared memory: 8
-// vectors at L = 36, Ltau = 359, complex64, 29.5 -> 21 us (complex128 52 -> 37);
-// 8 at 48 / 480, 54 -> 43 us.  With the rows of r asked for before the entries,
-// 26 us: a load that depends on another one waits for both behind the queue.
-// Four warps to a block: with eight, 25 us, the blocks' last wave being emptier.
+// What is left is loads in flight against the 60 MB of the first size below.
+// Device times, us, 8 vectors: with columns staged in shared memory, with the first
+// and the last form alone and shuffled entries, and now.  The builtin matrix, L = 36,
+// Ltau = 359: complex64 27.0, 17.6, 15.6, complex128 49.4, 34.5, 30.4; L = 48, Ltau =
+// 480, complex64: 50.9, 41.9, 38.3; there a diagonal 56.8, 112, 41.1, three taps
+// 67.0, 113, 42.0, 41 taps 256, 327, 235, a dense matrix 3211, 3085, 2421.  With the
+// rows of r asked for before the entries, a quarter more: a load that depends on
+// another one waits for both behind the queue.  Four warps to a block: with
+// eight, a fifth more, the blocks' last wave being emptier.
 template <typename R>
 struct Tap;  // a real tap times a complex number
 template <>

@@ -36,11 +36,11 @@
 // barrier to barrier and the exchange, the FMA chains and the loads add up.
 // Two and more blocks per SM overlap them, so the launch bounds (MaxT) trade
 // registers for co-resident blocks.  Taller tiles exchange less per site: M^dag M
-// of 8 complex64 vectors at L = 48, Ltau = 480 took 68 us with 2 x 2 tiles (56
-// registers, two 576-thread blocks per SM), 62 us with 2 x 4 and 56 us with
-// 2 x 6 (168 registers, two 192-thread blocks per SM; 1.15 warp instructions
-// per site against 1.68 of an engine that also exchanged phases and was
-// compiled per L, 72.5 us).
+// of 8 complex64 vectors at L = 48, Ltau = 480 takes 63 us on the device with 2 x 2
+// tiles (56 registers, two 576-thread blocks per SM), 76 us with 2 x 4 (one block of
+// nine warps per SM) and 55 us with 2 x 6 (168 registers, two 192-thread blocks per
+// SM; 1.15 warp instructions per site against 1.68 of an engine that also exchanged
+// phases and was compiled per L, 70 us).
 #pragma once
 
 #include <type_traits>
