@@ -36,9 +36,10 @@ class BondBond:
         self.Lx = self.Ly = Lx
         self.Ltau = Ltau
         self.chunk_bytes = int(chunk_bytes)
-        # pair sums in one pass: on the sides where that is faster (None), on
-        # every side that one of its kernels takes (True), on none (False)
-        self.fused = fused if fused is None else bool(fused)
+        # pair sums in one pass on the sides where that is faster; False: on none
+        # (complex128, L = 48, 12 vectors, one correlator: 3.2 ms in two passes, 9.9 in
+        # one with the kernel for any side)
+        self.fused = fused is None or bool(fused)
 
     # ---- helpers ----------------------------------------------------------
     def _chunk(self, ec, n_arrays=4):
@@ -53,7 +54,7 @@ class BondBond:
         back to real space; a_st, b_st are the fields of correlator ``kind``."""
         e, g, ep, pairs, S = inputs
         dt, nrv, Vs = e.dtype, e.shape[0], self.Lx * self.Ly
-        one = ops.bb_corr_lines(self.Lx, dt) if self.fused is None else self.fused
+        one = self.fused and ops.bb_corr_lines(self.Lx, dt)
         if one and ops.bb_corr(kind, e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
             S = S.view(self.Ly, self.Lx) / (Vs * Vs)
             return (torch.fft.ifft2(S, norm="forward") / (len(pairs) * self.Ltau)).to(dt)
@@ -156,8 +157,7 @@ class BondBond:
         vectors, complex64: 5.2 -> 1.5)."""
         e, g, ep, pairs, S = inputs = self._pair_inputs(eta, G_eta, boson)
         dt, Vs = e.dtype, self.Lx * self.Ly
-        if self.fused is not False and ops.bb_corr_sum(e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(),
-                                                       self.Lx, S):
+        if self.fused and ops.bb_corr_sum(e, g, ep, pairs[:, 0].contiguous(), pairs[:, 1].contiguous(), self.Lx, S):
             S = S.view(self.Ly, self.Lx) / (Vs * Vs)
             out = -(torch.fft.ifft2(S, norm="forward") / (len(pairs) * self.Ltau)).to(dt)
         else:
